@@ -249,6 +249,12 @@ int swd_rtm_batch(swd_ctx *ctx, int nshots, const swd_shot *shots, const float *
  *                 guards, CPML branches and strip code; 0: every block takes the general path.  The
  *                 same results bit for bit. */
 #define SWD_OPT_LEAN 12
+/* SWD_OPT_RESIDENT 1 (default): passes of one wavefield or of a pair (modelling with its twin, RTM
+ *                 with FP32 strips, batches at automatic size) on grids whose wavefields fit in the
+ *                 SMs' shared memory and registers run as one cooperative launch that keeps the
+ *                 fields on the chip between steps (stencil order 4, the other options at their
+ *                 defaults, no profiling).  The same results bit for bit.  0: the step kernels. */
+#define SWD_OPT_RESIDENT 13
 int swd_set_option(swd_ctx *ctx, int option, int value);
 int swd_get_option(swd_ctx *ctx, int option, int *value);
 

@@ -55,6 +55,13 @@ static Wave batch_wave(swd_ctx *c, int k)
     return w;
 }
 
+// Whether both passes of a survey's shot run on the chip (resident.cuh), one shot at a time.
+static bool batch_resident(const swd_ctx *c, ResPlan *f, ResPlan *b)
+{
+    return c->batch_opt == 0 && c->bwd_by_kind && c->image_blocks && c->strip_prec == SWD_STRIP_F32 &&
+           resident_plan(c, 1, f) && resident_plan(c, 2, b);
+}
+
 // One batch: shots[idx[0..nb)].  probe_steps > 0 runs only that many forward and backward
 // steps and skips the per-shot post (autotuner probes; the stack is left alone).
 static int rtm_batch_run(swd_ctx *ctx, const swd_shot *shots, const float *const *ricks, const float *const *data,
@@ -164,7 +171,21 @@ static int rtm_batch_run(swd_ctx *ctx, const swd_shot *shots, const float *const
     a.s0_mod = 1;
     a.bt = bt;
     const int nf = probe_steps > 0 ? std::min(probe_steps, ntmax) : ntmax;
-    {
+    // one shot whose wavefields fit on the chip: both passes as one launch each
+    ResPlan rp1, rp2;
+    bool ran = false;
+    if (nb == 1 && probe_steps <= 0 && batch_resident(ctx, &rp1, &rp2)) {
+        ResArgs r;
+        memset(&r, 0, sizeof r);
+        r.g = a.g; r.c = a.c; r.m = a.m;
+        r.w[0] = r.w[1] = a.w[0];
+        r.wav0 = r.wav1 = a.wav0;
+        r.sx = desc[0].sx; r.sz = desc[0].sz; r.nt = ntmax;
+        r.wells = a.wells; r.strips = st;
+        r.t0 = 0; r.nsteps = ntmax;
+        CKR(run_resident(ctx, r, rp1, 0, &ran));
+    }
+    if (!ran) {
         auto launch = [&](int k, cudaEvent_t *ev) {
             FwdArgs q = a;
             q.itoff = k;
@@ -195,7 +216,13 @@ static int rtm_batch_run(swd_ctx *ctx, const swd_shot *shots, const float *const
     bb.Sp = ctx->image_blocks ? F(ctx->bat.Sp) : nullptr;
     bb.bt = bt;
     const int nbk = probe_steps > 0 ? std::min(probe_steps, ntmax - 1) : ntmax - 1;
-    {
+    ran = false;
+    if (nb == 1 && probe_steps <= 0 && batch_resident(ctx, &rp1, &rp2)) {
+        bb.sx = desc[0].sx; bb.sz = desc[0].sz; bb.nt = ntmax;
+        ResArgs r = resident_bwd_args(bb, ntmax - 2, ntmax - 1);
+        CKR(run_resident(ctx, r, rp2, 1, &ran));
+    }
+    if (!ran) {
         const int by_kind = ctx->bwd_by_kind;
         auto launch = [&](int k, cudaEvent_t *ev) {
             BwdArgs q = bb;
@@ -224,7 +251,7 @@ static int rtm_batch_run(swd_ctx *ctx, const swd_shot *shots, const float *const
         k_max_nonneg<<<592, 256, 0, ctx->stream>>>(S, gb, mx);
         k_rtm_post<<<dim3((ctx->nz + 31) / 32, (ctx->nx + 7) / 8), dim3(32, 8), 0, ctx->stream>>>(
             I, S, F(ctx->vp), mx, ctx->ntx, ctx->ntz, ctx->ldz, ctx->pmlc, ctx->grid.dx, ctx->grid.dz, nullptr, nullptr,
-            nullptr, D(ctx->stack));
+            nullptr, D(ctx->stack), ctx->reserr.p ? I32(ctx->reserr) : nullptr);
         ctx->launches += 2;
     }
     CK(cudaGetLastError());
@@ -286,11 +313,23 @@ int swd_rtm_batch(swd_ctx *ctx, int nshots, const swd_shot *shots, const float *
     for (int i = 0; i < nshots; i++) order[i] = i;
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return shots[a].nt > shots[b].nt; });
     int B = ctx->batch_opt;
+    ResPlan rf, rb;
+    int done = 0;
+    if (batch_resident(ctx, &rf, &rb)) {
+        // one shot at a time; a pass that gave up has stacked nothing and runs again below
+        for (; done < nshots; done++) {
+            CKR(rtm_batch_run(ctx, shots, ricks, data, order.data() + done, 1, flags, 0));
+            CK(cudaStreamSynchronize(ctx->stream));
+            if (resident_failed(ctx)) break;
+        }
+        ctx->batch_tuned = 1;
+        B = 1;
+    }
     if (B <= 0) {
         if (ctx->batch_tuned <= 0) CKR(batch_autotune(ctx, shots, ricks, data, order.data(), nshots, flags, &ctx->batch_tuned));
         B = ctx->batch_tuned;
     }
-    for (int g = 0; g < nshots; g += B)
+    for (int g = done; g < nshots; g += B)
         CKR(rtm_batch_run(ctx, shots, ricks, data, order.data() + g, std::min(B, nshots - g), flags, 0));
     CK(cudaStreamSynchronize(ctx->stream));
     prof_collect(ctx);
@@ -345,6 +384,10 @@ int swd_set_option(swd_ctx *ctx, int option, int value)
                 tune_reset(ctx->tbwd, {0, 1, 4});
             }
             return SWD_OK;
+        case SWD_OPT_RESIDENT:
+            if (value != 0 && value != 1) return fail(ctx, SWD_ERR_ARG, "SWD_OPT_RESIDENT takes 0 or 1");
+            ctx->use_resident = value;
+            return SWD_OK;
         case SWD_OPT_LEAN:
             if (value != 0 && value != 1) return fail(ctx, SWD_ERR_ARG, "SWD_OPT_LEAN takes 0 or 1");
             ctx->use_lean = value;
@@ -368,6 +411,7 @@ int swd_get_option(swd_ctx *ctx, int option, int *value)
         case SWD_OPT_STAGED: *value = ctx->use_staged; return SWD_OK;
         case SWD_OPT_AUTOTUNE: *value = ctx->autotune; return SWD_OK;
         case SWD_OPT_LEAN: *value = ctx->use_lean; return SWD_OK;
+        case SWD_OPT_RESIDENT: *value = ctx->use_resident; return SWD_OK;
         case SWD_OPT_TUNED_FWD: *value = ctx->autotune && ctx->tfwd.choice >= 0 ? ctx->tfwd.cand[ctx->tfwd.choice] : -1; return SWD_OK;
         case SWD_OPT_TUNED_BWD: *value = ctx->autotune && ctx->tbwd.choice >= 0 ? ctx->tbwd.cand[ctx->tbwd.choice] : -1; return SWD_OK;
         default: return fail(ctx, SWD_ERR_ARG, "unknown option %d", option);

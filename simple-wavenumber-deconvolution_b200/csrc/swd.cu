@@ -12,6 +12,7 @@
 #include <algorithm>
 #include <initializer_list>
 #include <cmath>
+#include <mutex>
 #include <string>
 #include <utility>
 #include <vector>
@@ -20,6 +21,7 @@
 #include "prop.cuh"
 #include "prop_fused.cuh"
 #include "prop_tma.cuh"
+#include "resident.cuh"
 #include "born.cuh"
 #include "fft.cuh"
 #include "decon.cuh"
@@ -119,6 +121,14 @@ struct swd_ctx {
     size_t l2_bytes = 0;    // the device's L2 size, for the default register bounds
     int lean[4] = {0, 0, 0, 0};   // lean box of the step kernels (Geo::lx0 ...), from the CPML arrays
     int use_lean = 1;             // SWD_OPT_LEAN
+    // on-chip time loops (resident.cuh): exchange words, the tag of the last launch's last step,
+    // the error words (device, and the same flag in mapped host memory, read without a copy)
+    DevBuf resll, reserr;
+    unsigned res_epoch = 0;
+    volatile int *res_flag = nullptr;
+    int use_resident = 1;         // SWD_OPT_RESIDENT
+    int nsm = 0, coop = 0;
+    size_t smem_max = 0;
     // instrumentation
     int prof_every = 0;
     double prof_ms[SWD_NKERNELS] = {0};
@@ -131,7 +141,7 @@ struct swd_ctx {
     {
         DevBuf *all[] = {&vp, &rho, &dpdt, &wcol, &wmap, &seis, &seis2, &rdata, &colbuf, &kzcoef, &tw,
                          &strips, &strip_scale, &I, &S, &R, &stack, &reduce, &stage_in, &stage_out, &ctrl, &wav,
-                         &dk, &gk, &s0, &ckpt, &rbuf, &alias, &dpst, &dpsc, &cig, &cigring, &Ipart, &Spart, &Rpart};
+                         &dk, &gk, &s0, &ckpt, &rbuf, &alias, &resll, &reserr, &dpst, &dpsc, &cig, &cigring, &Ipart, &Spart, &Rpart};
         for (DevBuf *b : all) bufs.push_back(b);
         for (auto &b : adj) bufs.push_back(&b);
         for (auto &b : dcn) bufs.push_back(&b);
@@ -573,7 +583,8 @@ __global__ void k_max_nonneg(const double *__restrict__ a, size_t n, unsigned lo
 // grid, -vp^2 * (5-point Laplacian of In) on the interior, stacked in FP64.
 __global__ void k_rtm_post(const double *__restrict__ I, const double *__restrict__ S, const float *__restrict__ vp,
                            const unsigned long long *__restrict__ smax, int ntx, int ntz, int ldz, int pmlc,
-                           float dx, float dz, float *img_pp, float *img_src, float *fimage, double *stack)
+                           float dx, float dz, float *img_pp, float *img_src, float *fimage, double *stack,
+                           const int *skip)
 {
     const int nz = ntz - 2 * pmlc, nx = ntx - 2 * pmlc;
     const int iz = blockIdx.x * 32 + threadIdx.x, ixi = blockIdx.y * 8 + threadIdx.y;
@@ -594,7 +605,7 @@ __global__ void k_rtm_post(const double *__restrict__ I, const double *__restric
     if (img_pp) img_pp[o] = c;
     if (img_src) img_src[o] = (float)S[ip];
     if (fimage) fimage[o] = f;
-    if (stack) stack[o] += (double)f;
+    if (stack && !(skip && *skip)) stack[o] += (double)f;
 }
 
 // stacked image -> float, reference edge zeroing (acoustic_HLVSPRTMC.cpp:754-768)
@@ -1159,6 +1170,90 @@ static int run_steps(swd_ctx *ctx, swd_ctx::StepGraph &G, const void *key, size_
     return SWD_OK;
 }
 
+// ---- on-chip time loops (resident.cuh) ---------------------------------------------------
+// Whether the context's options ask for nothing but the default step kernels and the grid's
+// wavefields fit on the chip; plan receives the tiling for nw wavefields.  The plain kernels keep
+// every other case: larger grids, other stencil lengths, 16-bit strips, profiling, the kernel
+// variants the options select.
+static bool resident_plan(const swd_ctx *c, int nw, ResPlan *plan)
+{
+    if (!c->use_resident || !c->coop || c->Lc != RES_LC || c->path != SWD_PATH_PLAIN || !c->use_graphs || c->autotune ||
+        c->use_tma || c->use_staged || c->use_pdl || !c->use_lean || c->prof_every > 0)
+        return false;
+    return res_plan(c->ntx, c->ntz, c->nsm, c->smem_max, nw, plan);
+}
+
+// Two of these launches must not share the device (each would hold SMs the other waits for), so
+// every launch waits on the device for the previous one of this process: one event per device.
+struct ResGate {
+    std::mutex m;
+    cudaEvent_t ev = nullptr;
+};
+
+static ResGate &res_gate(int dev)
+{
+    static ResGate gates[64];
+    return gates[dev & 63];
+}
+
+// One pass of a.nsteps steps from a.t0.  *ran is false when the launch was refused (fewer SMs than
+// the device reports, say): the caller goes on with the plain kernels.  An error word that a kernel sets (a wait that gave up)
+// makes later launches return at once; resident_failed reads it after the stream has drained.
+static int run_resident(swd_ctx *ctx, ResArgs &a, const ResPlan &p, int mode, bool *ran)
+{
+    *ran = false;
+    const bool fresh = ctx->resll.n < p.ll_bytes || !ctx->resll.p || ctx->res_epoch > 0x7f000000u;
+    CKR(ensure(ctx, ctx->resll, p.ll_bytes));
+    if (fresh) {   // no stale word may carry a tag to come
+        CK(cudaMemsetAsync(ctx->resll.p, 0, ctx->resll.n, ctx->stream));
+        ctx->res_epoch = 0;
+    }
+    if (!ctx->reserr.p) {
+        CKR(ensure(ctx, ctx->reserr, 64));
+        CK(cudaMemsetAsync(ctx->reserr.p, 0, 64, ctx->stream));
+    }
+    if (!ctx->res_flag) {
+        void *h = nullptr;
+        CK(cudaHostAlloc(&h, 64, cudaHostAllocMapped));
+        memset(h, 0, 64);
+        ctx->res_flag = (volatile int *)h;
+    }
+    void *hd = nullptr;
+    CK(cudaHostGetDevicePointer(&hd, (void *)ctx->res_flag, 0));
+    a.ll = (uint4 *)ctx->resll.p;
+    a.err = I32(ctx->reserr);
+    a.host_err = (int *)hd;
+    a.TX = p.TX;
+    a.GX = p.GX;
+    a.GZ = p.GZ;
+    a.epoch = ctx->res_epoch;
+    ctx->res_epoch += (unsigned)a.nsteps + 1u;
+    ResGate &gate = res_gate(ctx->dev);
+    std::lock_guard<std::mutex> hold(gate.m);
+    if (!gate.ev) CK(cudaEventCreateWithFlags(&gate.ev, cudaEventDisableTiming));
+    else CK(cudaStreamWaitEvent(ctx->stream, gate.ev, 0));
+    if (res_launch(a, p, mode, ctx->stream) != cudaSuccess) {
+        cudaGetLastError();
+        ctx->use_resident = 0;
+        return SWD_OK;
+    }
+    CK(cudaEventRecord(gate.ev, ctx->stream));
+    ctx->launches++;
+    *ran = true;
+    return SWD_OK;
+}
+
+// After the stream has drained: whether a pass gave up.  The context then keeps to the plain
+// kernels, and the caller runs the pass again with them.
+static bool resident_failed(swd_ctx *ctx)
+{
+    if (!ctx->res_flag || !*ctx->res_flag) return false;
+    *ctx->res_flag = 0;
+    cudaMemsetAsync(ctx->reserr.p, 0, 64, ctx->stream);
+    ctx->use_resident = 0;
+    return true;
+}
+
 static int run_forward_fused(swd_ctx *ctx, FwdJob &J, ShotPlan &P);
 
 static int run_forward(swd_ctx *ctx, FwdJob &J, ShotPlan &P)
@@ -1221,6 +1316,23 @@ static int run_forward(swd_ctx *ctx, FwdJob &J, ShotPlan &P)
     a.wav0 = F(ctx->wav);
     a.wav1 = J.twin ? F(ctx->wav) + nt : F(ctx->wav);
     const int nw = J.twin ? 2 : 1;
+    // one field, or a field and its twin, whose grid fits on the chip: the whole pass in one launch
+    ResPlan rp;
+    if (!a.ck.every && !a.ds.buf && !a.s0_out && !a.dkappa && !a.dck && (!a.strips.buf || a.strips.prec == 0) &&
+        resident_plan(ctx, nw, &rp)) {
+        ResArgs r;
+        memset(&r, 0, sizeof r);
+        r.g = a.g; r.c = a.c; r.m = a.m;
+        r.w[0] = a.w[0]; r.w[1] = a.w[1];
+        r.wav0 = a.wav0; r.wav1 = a.wav1;
+        r.sx = a.sx; r.sz = a.sz; r.nt = nt;
+        r.wells = a.wells; r.seis = a.seis; r.colmap = a.colmap; r.colbuf = a.colbuf;
+        r.strips = a.strips;
+        r.t0 = 0; r.nsteps = nt;
+        bool ran;
+        CKR(run_resident(ctx, r, rp, 0, &ran));
+        if (ran) return SWD_OK;
+    }
     // one wavefield without checkpoints: the velocity kernel with TMA-staged pressure
     // the plain single-wavefield forward (RTM forward, modelling without a twin): variants of the
     // velocity and pressure launches, chosen by the tuner when SWD_OPT_AUTOTUNE is on
@@ -1537,6 +1649,16 @@ int swd_create(swd_ctx **out, const swd_grid *g)
         l2 = 0;
     }
     ctx->l2_bytes = (size_t)l2;
+    // what the on-chip time loops need; a failed query leaves them off
+    int smo = 0;
+    if (e == cudaSuccess &&
+        (cudaDeviceGetAttribute(&ctx->nsm, cudaDevAttrMultiProcessorCount, ctx->dev) != cudaSuccess ||
+         cudaDeviceGetAttribute(&ctx->coop, cudaDevAttrCooperativeLaunch, ctx->dev) != cudaSuccess ||
+         cudaDeviceGetAttribute(&smo, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->dev) != cudaSuccess)) {
+        cudaGetLastError();
+        ctx->coop = 0;
+    }
+    ctx->smem_max = (size_t)smo;
     if (e != cudaSuccess) {
         delete ctx;
         return SWD_ERR_CUDA;
@@ -1554,6 +1676,7 @@ int swd_destroy(swd_ctx *ctx)
         if (b->p) cudaFree(b->p);
     prof_collect(ctx);
     for (cudaEvent_t e : ctx->ev_pool) cudaEventDestroy(e);
+    if (ctx->res_flag) cudaFreeHost((void *)ctx->res_flag);
     graph_free(ctx->gfwd);
     graph_free(ctx->gbwd);
     graph_free(ctx->gseg);
@@ -1737,8 +1860,8 @@ int swd_set_strip_precision(swd_ctx *ctx, int prec)
     return SWD_OK;
 }
 
-int swd_forward(swd_ctx *ctx, const swd_shot *shot, const float *rick, const float *hrick, const float *kz_coef,
-                float *seis, float *seis_up, float *seis_down)
+static int forward_call(swd_ctx *ctx, const swd_shot *shot, const float *rick, const float *hrick, const float *kz_coef,
+                        float *seis, float *seis_up, float *seis_down)
 {
     CKR(check_ready(ctx));
     if (!rick || !seis) return fail(ctx, SWD_ERR_ARG, "rick and seis are required");
@@ -1785,6 +1908,13 @@ int swd_forward(swd_ctx *ctx, const swd_shot *shot, const float *rick, const flo
     CK(cudaStreamSynchronize(ctx->stream));
     prof_collect(ctx);
     return SWD_OK;
+}
+
+int swd_forward(swd_ctx *ctx, const swd_shot *shot, const float *rick, const float *hrick, const float *kz_coef,
+                float *seis, float *seis_up, float *seis_down)
+{
+    CKR(forward_call(ctx, shot, rick, hrick, kz_coef, seis, seis_up, seis_down));
+    return resident_failed(ctx) ? forward_call(ctx, shot, rick, hrick, kz_coef, seis, seis_up, seis_down) : SWD_OK;
 }
 
 int swd_set_scatter_model(swd_ctx *ctx, const float *vp1, const float *rho1)
@@ -1926,6 +2056,21 @@ static int rtm_forward_part(swd_ctx *ctx, const swd_shot *shot, const float *ric
     return SWD_OK;
 }
 
+// arguments of an on-chip backward pass of nsteps steps from it = t0 down
+static ResArgs resident_bwd_args(const BwdArgs &b, int t0, int nsteps)
+{
+    ResArgs r;
+    memset(&r, 0, sizeof r);
+    r.g = b.g; r.c = b.c; r.m = b.m;
+    r.w[0] = b.s; r.w[1] = b.r;
+    r.wav0 = b.wavsub;
+    r.sx = b.sx; r.sz = b.sz; r.nt = b.nt;
+    r.wells = b.wells; r.strips = b.strips; r.rdata = b.rdata;
+    r.I = b.I; r.S = b.S; r.Ip = b.Ip; r.Sp = b.Sp;
+    r.t0 = t0; r.nsteps = nsteps;
+    return r;
+}
+
 // RTM backward pass of the shot whose forward pass is kept: receiver data (-int int dt dt),
 // source reconstruction + receiver back-propagation + FP64 imaging, per-shot post and stack.
 static int rtm_backward_part(swd_ctx *ctx, const swd_shot *shot, const float *data, unsigned flags, float *image_pp,
@@ -2024,6 +2169,7 @@ static int rtm_backward_part(swd_ctx *ctx, const swd_shot *shot, const float *da
     b.Rp = blocks && ctx->have_R ? F(ctx->Rpart) : nullptr;
     const dim3 grid = grid_blocks(ctx);
     CKR(ensure(ctx, ctx->ctrl, 64));
+    const int *skip = nullptr;   // error word of an on-chip pass: its images are not stacked
     if (fz) {
         BStepArgs f;
         memset(&f, 0, sizeof f);
@@ -2073,6 +2219,16 @@ static int rtm_backward_part(swd_ctx *ctx, const swd_shot *shot, const float *da
     } else {
         b.itp = I32(ctx->ctrl);
         b.wavsub = F(ctx->wav);
+        ResPlan rp;
+        bool ran = false;
+        if (!want_cig && !ctx->have_R && blocks && ctx->bwd_by_kind && ctx->strip_prec == SWD_STRIP_F32 &&
+            resident_plan(ctx, 2, &rp)) {
+            ResArgs r = resident_bwd_args(b, nt - 2, nt - 1);
+            CKR(run_resident(ctx, r, rp, 1, &ran));
+        }
+        // (the error word also covers a forward pass that ran on the chip)
+        if (ctx->reserr.p) skip = I32(ctx->reserr);
+        if (!ran) {
         CigArgs cg;
         memset(&cg, 0, sizeof cg);
         if (want_cig) {
@@ -2145,6 +2301,7 @@ static int rtm_backward_part(swd_ctx *ctx, const swd_shot *shot, const float *da
         if (use_tma) CKR(tma_check(ctx));
         if (timing) tune_record(ctx->tbwd, pass_ms / (nt - 1));
         ctx->have_cig = want_cig;
+        }
     }
     CK(cudaGetLastError());
     // 4. per-shot post and stack
@@ -2161,7 +2318,7 @@ static int rtm_backward_part(swd_ctx *ctx, const swd_shot *shot, const float *da
     float *o_pp = F(ctx->stage_out), *o_src = o_pp + nimg, *o_f = o_src + nimg;
     k_rtm_post<<<dim3((ctx->nz + 31) / 32, (ctx->nx + 7) / 8), dim3(32, 8), 0, ctx->stream>>>(
         D(ctx->I), D(ctx->S), F(ctx->vp), (const unsigned long long *)ctx->reduce.p, ctx->ntx, ctx->ntz, ctx->ldz,
-        ctx->pmlc, ctx->grid.dx, ctx->grid.dz, o_pp, o_src, o_f, (flags & SWD_RTM_NO_STACK) ? nullptr : D(ctx->stack));
+        ctx->pmlc, ctx->grid.dx, ctx->grid.dz, o_pp, o_src, o_f, (flags & SWD_RTM_NO_STACK) ? nullptr : D(ctx->stack), skip);
     CK(cudaGetLastError());
     if (image_pp) CKR(from_dev(ctx, image_pp, o_pp, sizeof(float) * nimg));
     if (image_src) CKR(from_dev(ctx, image_src, o_src, sizeof(float) * nimg));
@@ -2178,6 +2335,9 @@ int swd_rtm_shot(swd_ctx *ctx, const swd_shot *shot, const float *rick, const fl
     CKR(check_ready(ctx));
     if (!rick || !data) return fail(ctx, SWD_ERR_ARG, "rick and data are required");
     CKR(rtm_forward_part(ctx, shot, rick, syn));
+    CKR(rtm_backward_part(ctx, shot, data, flags, image_pp, image_src, fimage));
+    if (!resident_failed(ctx)) return SWD_OK;
+    CKR(rtm_forward_part(ctx, shot, rick, syn));
     return rtm_backward_part(ctx, shot, data, flags, image_pp, image_src, fimage);
 }
 
@@ -2187,6 +2347,10 @@ int swd_rtm_forward(swd_ctx *ctx, const swd_shot *shot, const float *rick, float
     if (!rick) return fail(ctx, SWD_ERR_ARG, "rick is required");
     CKR(rtm_forward_part(ctx, shot, rick, syn));
     CK(cudaStreamSynchronize(ctx->stream));
+    if (resident_failed(ctx)) {
+        CKR(rtm_forward_part(ctx, shot, rick, syn));
+        CK(cudaStreamSynchronize(ctx->stream));
+    }
     prof_collect(ctx);
     return SWD_OK;
 }
@@ -2196,6 +2360,10 @@ int swd_rtm_backward(swd_ctx *ctx, const swd_shot *shot, const float *data, unsi
 {
     CKR(check_ready(ctx));
     if (!data) return fail(ctx, SWD_ERR_ARG, "data is required");
+    const swd_ctx::KeptShotState kept = ctx->kept;
+    CKR(rtm_backward_part(ctx, shot, data, flags, image_pp, image_src, fimage));
+    if (!resident_failed(ctx)) return SWD_OK;
+    ctx->kept = kept;   // a pass that gave up leaves the kept wavefield as it was
     return rtm_backward_part(ctx, shot, data, flags, image_pp, image_src, fimage);
 }
 

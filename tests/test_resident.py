@@ -1,0 +1,83 @@
+"""On-chip time loops (SWD_OPT_RESIDENT) against the step kernels: the same bits.
+
+The grids sit where the tiling can go wrong: one row or one column in the last tile, exactly full
+tiles, one tile only along z, the smallest grid, one and two columns per warp at the ends of their
+ranges, the largest grid that fits; receivers scattered over the whole padded grid (several per
+warp and per cell column, duplicates, frame cells), the source inside the strip band and in the
+frame.  The arithmetic is the same term by term, so the comparison is exact."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+# (nx, nz, pml): padded sizes are nx + 2 * (pml + 4)
+GRIDS = {
+    "smallest": (20, 20, 10),              # 48 x 48, one tile row, 8-column tiles
+    "z_full_tile": (100, 100, 10),         # 128 rows: exactly one tile
+    "z_one_row_left": (101, 101, 10),      # 129 x 129: last tile one row, last column tile one column
+    "x_13_columns": (620, 300, 10),        # 648 x 328: 13-column tiles, one column per warp, 16-warp kernel
+    "x_17_columns": (600, 400, 10),        # 628 x 428: two columns per warp, shortest
+    "x_24_columns": (850, 400, 15),        # 888 x 438: 24-column tiles, full
+}
+
+
+def _engine(swd, nx, nz, pml, nt, seed):
+    rng = np.random.default_rng(seed)
+    pmlc = pml + 4
+    v = (1900.0 + 900.0 * np.arange(nz)[None, :] / nz + rng.uniform(-80, 80, (nx, nz))).astype(np.float32)
+    vp = swd.pad_model(v, pmlc)
+    rho = (1000.0 + rng.uniform(-50, 50, vp.shape)).astype(np.float32)
+    E = swd.Engine(nx, nz, pml, 4, 5.0, 5.0, 5e-4, nt)
+    E.setup_default(vp, rho)
+    return E, rng, vp.shape
+
+
+@pytest.mark.parametrize("name", list(GRIDS))
+def test_resident_same_bits(swd, name):
+    nx, nz, pml = GRIDS[name]
+    nt = 150
+    E, rng, (ntx, ntz) = _engine(swd, nx, nz, pml, nt, 5)
+    pmlc = pml + 4
+    n = 60
+    rix, riz = rng.integers(0, ntx, n).astype(np.int32), rng.integers(0, ntz, n).astype(np.int32)
+    rix[:20] = pmlc + nx // 2          # a well, with two traces on one cell
+    riz[:20] = np.minimum(pmlc + np.arange(20), ntz - 1)
+    riz[1] = riz[0]
+    rick = swd.ricker_wave(nt, 25.0, 5e-4)
+    hr = E.hilbert(rick)
+    coef = rng.uniform(0.2, 1.0, swd.pow2(ntz)).astype(np.float32)
+    data = rng.standard_normal((n, nt)).astype(np.float32)
+    out = {}
+    for res in (0, 1):
+        E.set_option(swd.OPT_RESIDENT, res)
+        r = []
+        n0 = E.launch_count()
+        for sx, sz in ((pmlc + nx // 2, pmlc + 1), (3, ntz - 5)):
+            s = swd.ShotSpec(sx, sz, rix, riz, nt)
+            r.append(E.forward(s, rick))
+            r += list(E.forward(s, rick, hrick=hr, kz_coef=coef))
+            o = E.rtm_shot(s, rick, data, flags=swd.RTM_PREPROCESS | swd.RTM_NO_STACK, want=("image_pp", "image_src", "fimage", "syn"))
+            r += [o[k] for k in sorted(o)] + list(E.rtm_raw()[:2])
+            E.stack_reset()
+            E.rtm_batch([s, swd.ShotSpec(sx, sz, rix, riz, nt - 37)], [rick, rick[:nt - 37]], [data, data[:, :nt - 37].copy()])
+            r.append(E.stack(edge_zero=False))
+        out[res] = (r, E.launch_count() - n0)
+    assert E.get_option(swd.OPT_RESIDENT) == 1          # no pass gave up
+    assert out[1][1] < 0.1 * out[0][1]                  # and the time loops really ran as single launches
+    for i, (a, b) in enumerate(zip(out[1][0], out[0][0])):
+        assert i >= len(out[0][0]) // 2 or np.abs(b).max() > 0, i   # (the corner source is too far from some receivers)
+        assert np.array_equal(a, b), i
+
+
+def test_resident_needs_its_sizes(swd):
+    """A grid too large for the chip, another stencil length and 16-bit strips keep the step kernels."""
+    for nx, nz, Lc, prec in ((1200, 600, 4, 0), (100, 60, 3, 0), (100, 60, 4, 1)):
+        nt = 64
+        E = swd.Engine(nx, nz, 10, Lc, 5.0, 5.0, 5e-4, nt)
+        vp = np.full((nx + 2 * (10 + Lc), nz + 2 * (10 + Lc)), 2000.0, np.float32)
+        E.setup_default(vp, np.full_like(vp, 1000.0))
+        E.set_strip_precision(prec)
+        s = swd.ShotSpec(30, 30, np.array([40], np.int32), np.array([30], np.int32), nt)
+        n0 = E.launch_count()
+        E.rtm_forward(s, swd.ricker_wave(nt, 25.0, 5e-4))
+        assert E.launch_count() - n0 >= 2 * nt
