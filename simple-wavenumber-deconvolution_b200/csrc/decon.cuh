@@ -83,6 +83,47 @@ __device__ __forceinline__ float img_at(const float *__restrict__ im, int nx, in
     return __ldg(im + (size_t)ix * nz + iz);
 }
 
+// The PSF of window w: the nearest lattice point (indices clamped to [3, nwpsf-4], :586-598) and,
+// with psf_interp, the four lattice points around the window centre and their weights.
+struct PsfPick {
+    int ixf, izf;
+    int fx0, fx1, fz0, fz1;
+    double tx, tz;
+};
+
+__device__ __forceinline__ PsfPick psf_pick(const DeconGeo &g, int w)
+{
+    PsfPick q;
+    const int ix = g.stepwinx * (w / g.stepnumz), iz = g.stepwinz * (w % g.stepnumz);
+    q.ixf = (ix - g.halfpsfwx) / g.psfwinx;
+    q.izf = (iz - g.halfpsfwz) / g.psfwinz;
+    if (q.ixf <= 2) q.ixf = 3;
+    if (q.ixf >= g.nxwpsf - 3) q.ixf = g.nxwpsf - 4;
+    if (q.izf <= 2) q.izf = 3;
+    if (q.izf >= g.nzwpsf - 3) q.izf = g.nzwpsf - 4;
+    q.fx0 = q.fx1 = q.fz0 = q.fz1 = 0;
+    q.tx = q.tz = 0.0;
+    if (g.psf_interp) {
+        psf_bracket(ix, g.halfpsfwx, g.psfwinx, g.nxwpsf, q.fx0, q.fx1, q.tx);
+        psf_bracket(iz, g.halfpsfwz, g.psfwinz, g.nzwpsf, q.fz0, q.fz1, q.tz);
+    }
+    return q;
+}
+
+// PSF patch value at (ixx, izz): of the nearest lattice point, or the bilinear blend of the four,
+// formed in double without contraction and rounded to float
+__device__ __forceinline__ float psf_value(const DeconGeo &g, const PsfPick &q, const float *__restrict__ psf, int ixx, int izz)
+{
+    if (!g.psf_interp) return img_at(psf, g.nx, g.nz, q.ixf * g.psfwinx + ixx, q.izf * g.psfwinz + izz);
+    const int xa = q.fx0 * g.psfwinx + ixx, xb = q.fx1 * g.psfwinx + ixx;
+    const int za = q.fz0 * g.psfwinz + izz, zb = q.fz1 * g.psfwinz + izz;
+    const double a = img_at(psf, g.nx, g.nz, xa, za), b = img_at(psf, g.nx, g.nz, xb, za);
+    const double c = img_at(psf, g.nx, g.nz, xa, zb), d = img_at(psf, g.nx, g.nz, xb, zb);
+    const double s1 = __dadd_rn(__dmul_rn(1.0 - q.tx, a), __dmul_rn(q.tx, b));
+    const double s2 = __dadd_rn(__dmul_rn(1.0 - q.tx, c), __dmul_rn(q.tx, d));
+    return (float)__dadd_rn(__dmul_rn(1.0 - q.tz, s1), __dmul_rn(q.tz, s2));
+}
+
 __device__ void dft2(float2 *s, const WfftPlan &P0, const WfftPlan &P1, int n0, int n1, int sign)
 {
     fft_pass(s, P1, n0, 1, n1, sign);   // rows (length n1)
@@ -228,31 +269,7 @@ __device__ void decon_window(const DeconGeo &g, const float *__restrict__ mig, c
     __shared__ unsigned s_fmax;
     const int ix = g.stepwinx * (w / g.stepnumz), iz = g.stepwinz * (w % g.stepnumz);
     const int tid = threadIdx.x, nthr = blockDim.x;
-    // nearest PSF on the lattice, indices clamped to [3, nwpsf-4] (:586-598)
-    int ixf = (ix - g.halfpsfwx) / g.psfwinx, izf = (iz - g.halfpsfwz) / g.psfwinz;
-    if (ixf <= 2) ixf = 3;
-    if (ixf >= g.nxwpsf - 3) ixf = g.nxwpsf - 4;
-    if (izf <= 2) izf = 3;
-    if (izf >= g.nzwpsf - 3) izf = g.nzwpsf - 4;
-    const int ixp = g.halfpsfwx + ixf * g.psfwinx, izp = g.halfpsfwz + izf * g.psfwinz;
-    // PSF patch value: the nearest lattice PSF, or (psf_interp) the bilinear blend of the four
-    // around the window centre, formed in double without contraction and rounded to float
-    int fx0 = 0, fx1 = 0, fz0 = 0, fz1 = 0;
-    double tx = 0.0, tz = 0.0;
-    if (g.psf_interp) {
-        psf_bracket(ix, g.halfpsfwx, g.psfwinx, g.nxwpsf, fx0, fx1, tx);
-        psf_bracket(iz, g.halfpsfwz, g.psfwinz, g.nzwpsf, fz0, fz1, tz);
-    }
-    auto psf_val = [&](int ixx, int izz) -> float {
-        if (!g.psf_interp) return img_at(psf, g.nx, g.nz, ixp + ixx - g.halfpsfwx, izp + izz - g.halfpsfwz);
-        const int xa = fx0 * g.psfwinx + ixx, xb = fx1 * g.psfwinx + ixx;
-        const int za = fz0 * g.psfwinz + izz, zb = fz1 * g.psfwinz + izz;
-        const double a = img_at(psf, g.nx, g.nz, xa, za), b = img_at(psf, g.nx, g.nz, xb, za);
-        const double c = img_at(psf, g.nx, g.nz, xa, zb), d = img_at(psf, g.nx, g.nz, xb, zb);
-        const double s1 = __dadd_rn(__dmul_rn(1.0 - tx, a), __dmul_rn(tx, b));
-        const double s2 = __dadd_rn(__dmul_rn(1.0 - tx, c), __dmul_rn(tx, d));
-        return (float)__dadd_rn(__dmul_rn(1.0 - tz, s1), __dmul_rn(tz, s2));
-    };
+    const PsfPick pick = psf_pick(g, w);
 
     for (int j = tid; j < n; j += nthr) Z[j] = make_float2(0.f, 0.f);
     if (tid == 64) s_fmax = 0u;
@@ -266,7 +283,7 @@ __device__ void decon_window(const DeconGeo &g, const float *__restrict__ mig, c
     }
     for (int j = tid; j < g.psfwinx * g.psfwinz; j += nthr) {
         const int ixx = j / g.psfwinz, izz = j % g.psfwinz;
-        Z[ixx * g.FZ + izz].y = psf_val(ixx, izz);
+        Z[ixx * g.FZ + izz].y = psf_value(g, pick, psf, ixx, izz);
     }
     __syncthreads();
     // L1 norms in the reference's order and rounding (:554-576, :618-620), from the buffer:

@@ -25,6 +25,7 @@
 #include "born.cuh"
 #include "fft.cuh"
 #include "decon.cuh"
+#include "decon_dense.cuh"
 
 using namespace swd;
 
@@ -1580,6 +1581,73 @@ static cudaError_t launch_decon_windows(const DeconGeo &g, const float *mig, con
     return cudaGetLastError();
 }
 
+// Plan of the dense path (decon_dense.cuh) for a geometry; false when it does not apply: the
+// iterative option (its loop transforms whole buffers), transforms taken over a transposed view of
+// the buffer (n0 x n1 != FX x FZ: the patches are no rectangles there), windows whose parts and
+// tables do not fit in shared memory.
+static bool dense_plan(const DeconGeo &g, DenseGeo &d)
+{
+    memset(&d, 0, sizeof d);
+    if (g.iters > 0 || g.n0 != g.FX || g.n1 != g.FZ) return false;
+    d.L1 = g.n0; d.L2 = g.n1;
+    d.K1 = d.L1 / 2 + 1; d.K2 = d.L2 / 2 + 1;
+    d.hm1 = g.halfltwx; d.hm2 = g.halfltwz; d.hp1 = g.halfpsfwx; d.hp2 = g.halfpsfwz;
+    d.ho1 = g.halfoutwx; d.ho2 = g.halfoutwz;
+    d.K1p = up4(d.K1); d.R1p = up4(d.ho1 + 1); d.R2p = up8(d.ho2 + 1);
+    d.TR1 = up8(std::max(d.hm1 + 1, d.R1p));
+    d.TR2 = up8(std::max(d.hm2 + 1, d.R2p));
+    if (d.L1 == d.L2) d.TR1 = d.TR2 = std::max(d.TR1, d.TR2);
+    // columns per block: as many as leave room for two CTAs on an SM, or for one
+    const size_t cap[2] = {113 * 1024, 226 * 1024};
+    for (int c = 0; c < 2; c++)
+        for (int nb = 1; nb <= (d.K2 + 7) / 8; nb++) {
+            d.NB = nb;
+            d.blk = up8((d.K2 + nb - 1) / nb);
+            if (d.blk > 40) continue;
+            d.yp = odd4(d.blk);
+            d.KT1 = odd4(std::max(d.K1p, d.L1 == d.L2 ? nb * d.blk : 0));
+            d.KT2 = d.L1 == d.L2 ? d.KT1 : odd4(nb * d.blk);
+            if (dense_smem(d, d.hm1, d.hm2) > cap[c] || (c == 0 && d.blk < 16)) continue;
+            const int tiles = 4 * (d.R1p / 4) * (d.R2p / 8);
+            d.nthr = c == 0 ? 256 : 512;
+            d.tiles = 1;
+            if (tiles > d.nthr) { d.tiles = 2; d.nthr = 384; }
+            if (tiles > d.tiles * d.nthr) return false;
+            // one PSF per lattice point that windows can use, or per window where that is fewer
+            const long long nl = (long long)(g.nxwpsf - 6) * (g.nzwpsf - 6);
+            d.pz = g.psf_interp || nl > g.totalnum ? 0 : g.nzwpsf - 6;
+            d.npsf = d.pz ? (int)nl : g.totalnum;
+            return true;
+        }
+    return false;
+}
+
+// floats of scratch of the dense path: spectra, maxima, tables
+static size_t dense_scratch(const DenseGeo &d)
+{
+    return 4 * dense_spec(d) * d.npsf + (((size_t)d.npsf + 63) & ~(size_t)63) + dense_tab_len(d);
+}
+
+// Window kernels of the dense path over the scratch ws; *launches counts them.
+static cudaError_t launch_decon_dense(const DeconGeo &g, const DenseGeo &d, const float *mig, const float *psf, float *winout,
+                                      float *ws, cudaStream_t st, int *launches)
+{
+    float4 *spec = (float4 *)ws;
+    float *smax = ws + 4 * dense_spec(d) * d.npsf, *tabs = smax + (((size_t)d.npsf + 63) & ~(size_t)63);
+    k_dense_tables<<<(d.TR1 * d.KT1 + 127) / 128, 128, 0, st>>>(tabs, d.L1, d.K1, d.TR1, d.KT1);
+    if (d.L1 != d.L2) k_dense_tables<<<(d.TR2 * d.KT2 + 127) / 128, 128, 0, st>>>(tabs + dense_tab1(d), d.L2, d.K2, d.TR2, d.KT2);
+    *launches = d.L1 != d.L2 ? 4 : 3;
+    const size_t sp = dense_smem(d, d.hp1, d.hp2), sm = dense_smem(d, d.hm1, d.hm2);
+    const void *fn = d.tiles == 1 ? (const void *)k_dense_window<1> : (const void *)k_dense_window<2>;
+    cudaError_t e = cudaFuncSetAttribute(k_dense_psf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sp);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    if (e != cudaSuccess) return e;
+    k_dense_psf<<<d.npsf, 256, sp, st>>>(g, d, psf, spec, smax, tabs);
+    if (d.tiles == 1) k_dense_window<1><<<g.totalnum, d.nthr, sm, st>>>(g, d, mig, spec, smax, winout, tabs);
+    else k_dense_window<2><<<g.totalnum, d.nthr, sm, st>>>(g, d, mig, spec, smax, winout, tabs);
+    return cudaGetLastError();
+}
+
 // ------------------------------------------------------------------------------------
 // Static scratch of swd_decon_noalloc: the per-window result slots and the output taper of
 // one deconvolution, so that entry point never allocates.  Every device that loads this
@@ -2541,9 +2609,16 @@ int swd_decon(swd_ctx *ctx_in, const swd_decon_params *p, const float *migreal, 
         const bool dout = is_device_ptr_on(mig_dec, ctx->dev) && is_device_ptr_on(mig_coef, ctx->dev);
         DevBuf &bin = ctx->dcn[0], &bcoef = ctx->dcn[1], &bwin = ctx->dcn[2], &bout = ctx->dcn[3], &bws = ctx->dcn[4],
                &btab = ctx->dcn[5];
-        const int nblk = decon_persistent(g) ? decon_ws_blocks(g, ctx->dev) : 0;
-        if (decon_persistent(g) && nblk < 1) { rc = fail(ctx, SWD_ERR_CUDA, "decon: no launch shape for the window kernel"); break; }
-        if (decon_persistent(g)) rc = ensure(ctx, bws, sizeof(float) * (size_t)nblk * decon_ws_floats(g));
+        // the dense path where it applies and its scratch can be had, else the FFT windows
+        DenseGeo dg;
+        bool dense = dense_plan(g, dg);
+        if (dense && ensure(ctx, bws, sizeof(float) * dense_scratch(dg)) != SWD_OK) {
+            cudaGetLastError();
+            dense = false;
+        }
+        const int nblk = !dense && decon_persistent(g) ? decon_ws_blocks(g, ctx->dev) : 0;
+        if (!dense && decon_persistent(g) && nblk < 1) { rc = fail(ctx, SWD_ERR_CUDA, "decon: no launch shape for the window kernel"); break; }
+        if (!dense && decon_persistent(g)) rc = ensure(ctx, bws, sizeof(float) * (size_t)nblk * decon_ws_floats(g));
         if (!rc && !din) rc = ensure(ctx, bin, sizeof(float) * 2 * np);
         if (!rc) rc = ensure(ctx, bcoef, sizeof(float) * nout);
         if (!rc) rc = ensure(ctx, bwin, sizeof(float) * nout * g.totalnum);
@@ -2556,13 +2631,15 @@ int swd_decon(swd_ctx *ctx_in, const swd_decon_params *p, const float *migreal, 
         if (!rc && cudaMemcpyAsync(bcoef.p, coefr.data(), sizeof(float) * nout, cudaMemcpyHostToDevice, ctx->stream) != cudaSuccess)
             rc = fail(ctx, SWD_ERR_CUDA, "decon: coefficient upload");
         if (!rc) {
-            cudaError_t e = launch_decon_windows(g, im, ps, F(bwin), F(bws), nblk, (float2 *)btab.p, ctx->stream);
+            int nl = g.n1 != g.n0 ? 3 : 2;
+            cudaError_t e = dense ? launch_decon_dense(g, dg, im, ps, F(bwin), F(bws), ctx->stream, &nl)
+                                  : launch_decon_windows(g, im, ps, F(bwin), F(bws), nblk, (float2 *)btab.p, ctx->stream);
             if (e == cudaSuccess) {
                 k_decon_gather<<<592, 256, 0, ctx->stream>>>(g, F(bwin), F(bcoef), od, oc);
                 e = cudaGetLastError();
             }
             if (e != cudaSuccess) rc = fail(ctx, SWD_ERR_CUDA, "decon kernels: %s", cudaGetErrorString(e));
-            else ctx->launches += g.n1 != g.n0 ? 4 : 3;
+            else ctx->launches += nl + 1;
         }
         if (!rc && !dout) rc = from_dev(ctx, mig_dec, od, sizeof(float) * np);
         if (!rc && !dout) rc = from_dev(ctx, mig_coef, oc, sizeof(float) * np);
