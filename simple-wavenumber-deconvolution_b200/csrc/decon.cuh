@@ -418,36 +418,36 @@ __global__ void __launch_bounds__(512) k_decon_window_ws(DeconGeo g, const float
 }
 
 // Overlap-add of the window slots in window order (:656-673), float accumulators with the
-// reference's double-then-round update, cropped to nx x nz (:724-731).
-__global__ void k_decon_gather(DeconGeo g, const float *__restrict__ winout, const float *__restrict__ coefr,
-                               float *__restrict__ dec, float *__restrict__ coef)
+// reference's double-then-round update, cropped to nx x nz (:724-731).  One block row per image
+// column (blockIdx.x = px), so the window ranges along x are uniform and no 64-bit division is
+// left (4001 x 1601: 104 -> 77 us, cold cache).
+constexpr int GATHER_NTHR = 256;
+__global__ void __launch_bounds__(GATHER_NTHR) k_decon_gather(DeconGeo g, const float *__restrict__ winout, const float *__restrict__ coefr,
+                                                              float *__restrict__ dec, float *__restrict__ coef)
 {
-    const size_t np = (size_t)g.nx * g.nz;
+    const int px = blockIdx.x, pz = blockIdx.y * GATHER_NTHR + threadIdx.x;
+    if (pz >= g.nz) return;
     const int nout = g.outwinx * g.outwinz;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < np; i += (size_t)gridDim.x * blockDim.x) {
-        const int px = (int)(i / g.nz), pz = (int)(i % g.nz);
-        // windows a (x) with a*stepwinx - halfoutwx <= px <= a*stepwinx - halfoutwx + outwinx - 1
-        int alo = px + g.halfoutwx - g.outwinx + 1;
-        alo = alo <= 0 ? 0 : (alo + g.stepwinx - 1) / g.stepwinx;
-        int ahi = (px + g.halfoutwx) / g.stepwinx;
-        if (ahi > g.stepnumx - 1) ahi = g.stepnumx - 1;
-        int blo = pz + g.halfoutwz - g.outwinz + 1;
-        blo = blo <= 0 ? 0 : (blo + g.stepwinz - 1) / g.stepwinz;
-        int bhi = (pz + g.halfoutwz) / g.stepwinz;
-        if (bhi > g.stepnumz - 1) bhi = g.stepnumz - 1;
-        float acc = 0.f, cacc = 0.f;
-        for (int a = alo; a <= ahi; a++)
-            for (int b = blo; b <= bhi; b++) {
-                const int ixx = px - (a * g.stepwinx - g.halfoutwx), izz = pz - (b * g.stepwinz - g.halfoutwz);
-                const int ipc = ixx * g.outwinz + izz;
-                const float cr = __ldg(coefr + ipc);
-                const float v = winout[(size_t)(a * g.stepnumz + b) * nout + ipc];
-                acc = (float)((double)acc + (double)v * (double)cr);
-                cacc = cacc + cr;
-            }
-        dec[i] = acc;
-        coef[i] = cacc;
-    }
+    // windows a (x) with a*stepwinx - halfoutwx <= px <= a*stepwinx - halfoutwx + outwinx - 1
+    int alo = px + g.halfoutwx - g.outwinx + 1;
+    alo = alo <= 0 ? 0 : (alo + g.stepwinx - 1) / g.stepwinx;
+    const int ahi = min((px + g.halfoutwx) / g.stepwinx, g.stepnumx - 1);
+    int blo = pz + g.halfoutwz - g.outwinz + 1;
+    blo = blo <= 0 ? 0 : (blo + g.stepwinz - 1) / g.stepwinz;
+    const int bhi = min((pz + g.halfoutwz) / g.stepwinz, g.stepnumz - 1);
+    float acc = 0.f, cacc = 0.f;
+    for (int a = alo; a <= ahi; a++)
+        for (int b = blo; b <= bhi; b++) {
+            const int ixx = px - (a * g.stepwinx - g.halfoutwx), izz = pz - (b * g.stepwinz - g.halfoutwz);
+            const int ipc = ixx * g.outwinz + izz;
+            const float cr = __ldg(coefr + ipc);
+            const float v = __ldg(winout + (size_t)(a * g.stepnumz + b) * nout + ipc);
+            acc = (float)((double)acc + (double)v * (double)cr);
+            cacc = cacc + cr;
+        }
+    const size_t i = (size_t)px * g.nz + pz;
+    dec[i] = acc;
+    coef[i] = cacc;
 }
 
 }  // namespace swd

@@ -1527,6 +1527,8 @@ static int decon_geo(const swd_decon_params *p, DeconGeo &g)
     return SWD_OK;
 }
 
+static dim3 gather_grid(const DeconGeo &g) { return dim3(g.nx, (g.nz + GATHER_NTHR - 1) / GATHER_NTHR); }
+
 // Launch shape of the persistent window kernel (staged transforms or the iterative option): a
 // 96 KB shared chunk when staged, else the buffer in shared memory; as many CTAs as are
 // resident at once, each owning decon_ws_floats(g) floats of workspace.
@@ -1642,7 +1644,7 @@ static cudaError_t launch_decon_dense(const DeconGeo &g, const DenseGeo &d, cons
     cudaError_t e = cudaFuncSetAttribute(k_dense_psf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sp);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     if (e != cudaSuccess) return e;
-    k_dense_psf<<<d.npsf, 256, sp, st>>>(g, d, psf, spec, smax, tabs);
+    k_dense_psf<<<d.npsf, 2 * (sp + 1024) <= 227 * 1024 ? 256 : 512, sp, st>>>(g, d, psf, spec, smax, tabs);
     if (d.tiles == 1) k_dense_window<1><<<g.totalnum, d.nthr, sm, st>>>(g, d, mig, spec, smax, winout, tabs);
     else k_dense_window<2><<<g.totalnum, d.nthr, sm, st>>>(g, d, mig, spec, smax, winout, tabs);
     return cudaGetLastError();
@@ -2635,7 +2637,7 @@ int swd_decon(swd_ctx *ctx_in, const swd_decon_params *p, const float *migreal, 
             cudaError_t e = dense ? launch_decon_dense(g, dg, im, ps, F(bwin), F(bws), ctx->stream, &nl)
                                   : launch_decon_windows(g, im, ps, F(bwin), F(bws), nblk, (float2 *)btab.p, ctx->stream);
             if (e == cudaSuccess) {
-                k_decon_gather<<<592, 256, 0, ctx->stream>>>(g, F(bwin), F(bcoef), od, oc);
+                k_decon_gather<<<gather_grid(g), GATHER_NTHR, 0, ctx->stream>>>(g, F(bwin), F(bcoef), od, oc);
                 e = cudaGetLastError();
             }
             if (e != cudaSuccess) rc = fail(ctx, SWD_ERR_CUDA, "decon kernels: %s", cudaGetErrorString(e));
@@ -2704,7 +2706,7 @@ int swd_decon_noalloc(const swd_decon_params *p, const float *migreal, const flo
     if (launch_decon_windows(g, migreal, migpsf, winout, coefr + wsoff, nblk, (float2 *)(coefr + tabof), st) !=
         cudaSuccess)
         return SWD_ERR_CUDA;
-    k_decon_gather<<<592, 256, 0, st>>>(g, winout, coefr, mig_dec, mig_coef);
+    k_decon_gather<<<gather_grid(g), GATHER_NTHR, 0, st>>>(g, winout, coefr, mig_dec, mig_coef);
     return cudaGetLastError() == cudaSuccess ? SWD_OK : SWD_ERR_CUDA;
 }
 
