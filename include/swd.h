@@ -255,6 +255,11 @@ int swd_rtm_batch(swd_ctx *ctx, int nshots, const swd_shot *shots, const float *
  *                 fields on the chip between steps (stencil order 4, the other options at their
  *                 defaults, no profiling).  The same results bit for bit.  0: the step kernels. */
 #define SWD_OPT_RESIDENT 13
+/* SWD_OPT_MARCH 1 (default): on grids whose fields fill the device's L2, the forward passes of one
+ *                 wavefield (RTM, modelling without a twin) run each time step as one sweep along x
+ *                 that makes both half steps (stencil order 4, the other options at their defaults,
+ *                 no profiling).  The same results bit for bit.  0: the step kernels. */
+#define SWD_OPT_MARCH 14
 int swd_set_option(swd_ctx *ctx, int option, int value);
 int swd_get_option(swd_ctx *ctx, int option, int *value);
 

@@ -384,6 +384,10 @@ int swd_set_option(swd_ctx *ctx, int option, int value)
                 tune_reset(ctx->tbwd, {0, 1, 4});
             }
             return SWD_OK;
+        case SWD_OPT_MARCH:
+            if (value != 0 && value != 1) return fail(ctx, SWD_ERR_ARG, "SWD_OPT_MARCH takes 0 or 1");
+            ctx->use_march = value;
+            return SWD_OK;
         case SWD_OPT_RESIDENT:
             if (value != 0 && value != 1) return fail(ctx, SWD_ERR_ARG, "SWD_OPT_RESIDENT takes 0 or 1");
             ctx->use_resident = value;
@@ -411,6 +415,7 @@ int swd_get_option(swd_ctx *ctx, int option, int *value)
         case SWD_OPT_STAGED: *value = ctx->use_staged; return SWD_OK;
         case SWD_OPT_AUTOTUNE: *value = ctx->autotune; return SWD_OK;
         case SWD_OPT_LEAN: *value = ctx->use_lean; return SWD_OK;
+        case SWD_OPT_MARCH: *value = ctx->use_march; return SWD_OK;
         case SWD_OPT_RESIDENT: *value = ctx->use_resident; return SWD_OK;
         case SWD_OPT_TUNED_FWD: *value = ctx->autotune && ctx->tfwd.choice >= 0 ? ctx->tfwd.cand[ctx->tfwd.choice] : -1; return SWD_OK;
         case SWD_OPT_TUNED_BWD: *value = ctx->autotune && ctx->tbwd.choice >= 0 ? ctx->tbwd.cand[ctx->tbwd.choice] : -1; return SWD_OK;

@@ -22,6 +22,7 @@
 #include "prop_fused.cuh"
 #include "prop_tma.cuh"
 #include "resident.cuh"
+#include "march.cuh"
 #include "born.cuh"
 #include "fft.cuh"
 #include "decon.cuh"
@@ -128,6 +129,8 @@ struct swd_ctx {
     unsigned res_epoch = 0;
     volatile int *res_flag = nullptr;
     int use_resident = 1;         // SWD_OPT_RESIDENT
+    int use_march = 1;            // SWD_OPT_MARCH
+    DevBuf marchl, marcht, marchr;   // strip blocks, tasks, ring of FP32 strips of a marching pass
     int nsm = 0, coop = 0;
     size_t smem_max = 0;
     // instrumentation
@@ -142,7 +145,7 @@ struct swd_ctx {
     {
         DevBuf *all[] = {&vp, &rho, &dpdt, &wcol, &wmap, &seis, &seis2, &rdata, &colbuf, &kzcoef, &tw,
                          &strips, &strip_scale, &I, &S, &R, &stack, &reduce, &stage_in, &stage_out, &ctrl, &wav,
-                         &dk, &gk, &s0, &ckpt, &rbuf, &alias, &resll, &reserr, &dpst, &dpsc, &cig, &cigring, &Ipart, &Spart, &Rpart};
+                         &dk, &gk, &s0, &ckpt, &rbuf, &alias, &resll, &reserr, &marchl, &marcht, &marchr, &dpst, &dpsc, &cig, &cigring, &Ipart, &Spart, &Rpart};
         for (DevBuf *b : all) bufs.push_back(b);
         for (auto &b : adj) bufs.push_back(&b);
         for (auto &b : dcn) bufs.push_back(&b);
@@ -1171,6 +1174,12 @@ static int run_steps(swd_ctx *ctx, swd_ctx::StepGraph &G, const void *key, size_
     return SWD_OK;
 }
 
+// Whether the context's options ask for nothing but the default step kernels (with graphs or not).
+static bool default_steps(const swd_ctx *c)
+{
+    return c->path == SWD_PATH_PLAIN && !c->autotune && !c->use_tma && !c->use_staged && !c->use_pdl && c->use_lean && c->prof_every == 0;
+}
+
 // ---- on-chip time loops (resident.cuh) ---------------------------------------------------
 // Whether the context's options ask for nothing but the default step kernels and the grid's
 // wavefields fit on the chip; plan receives the tiling for nw wavefields.  The plain kernels keep
@@ -1178,9 +1187,7 @@ static int run_steps(swd_ctx *ctx, swd_ctx::StepGraph &G, const void *key, size_
 // variants the options select.
 static bool resident_plan(const swd_ctx *c, int nw, ResPlan *plan)
 {
-    if (!c->use_resident || !c->coop || c->Lc != RES_LC || c->path != SWD_PATH_PLAIN || !c->use_graphs || c->autotune ||
-        c->use_tma || c->use_staged || c->use_pdl || !c->use_lean || c->prof_every > 0)
-        return false;
+    if (!c->use_resident || !c->coop || c->Lc != RES_LC || !c->use_graphs || !default_steps(c)) return false;
     return res_plan(c->ntx, c->ntz, c->nsm, c->smem_max, nw, plan);
 }
 
@@ -1253,6 +1260,135 @@ static bool resident_failed(swd_ctx *ctx)
     cudaMemsetAsync(ctx->reserr.p, 0, 64, ctx->stream);
     ctx->use_resident = 0;
     return true;
+}
+
+// Whether the one-wavefield forward passes run as marches (march.cuh): grids whose six arrays of a
+// step (p, vx, vz, three coefficients) take more than 0.8 of the L2 (4.5 M cells: 37.9 -> 34.1 us per
+// step; 3.3 M cells, 0.63 of it: 24.6 -> 25.3), in streams that can be captured (16-bit strips are
+// encoded once per captured chunk).
+static bool march_ok(const swd_ctx *c)
+{
+    return c->use_march && c->Lc == MARCH_LC && default_steps(c) && c->use_graphs && c->stream &&
+           (double)c->ntx * c->ldz * sizeof(float) * 6 > 0.8 * (double)c->l2_bytes;
+}
+
+// Tasks of a march: row tiles x column chunks, those that touch the frame (guards, CPML terms: about
+// twice the instructions per column) in narrow chunks and first, so that they end with the others.
+static void march_tasks_of(const swd_ctx *c, std::vector<int4> &t, int wide, int narrow, const std::vector<int> &wcol, size_t *lean_tasks)
+{
+    const int gz = (c->ntz + MARCH_OWN - 1) / MARCH_OWN, lx0 = c->lean[0], lx1 = c->lean[1], lz0 = c->lean[2], lz1 = c->lean[3];
+    std::vector<int4> in;
+    for (int bz = 0; bz < gz; bz++) {
+        const int zb = bz * MARCH_OWN - 8;
+        const bool zl = zb >= lz0 && zb + 128 <= lz1;
+        for (int x = 0; x < c->ntx;) {
+            const bool lean = zl && x - 8 >= lx0 && x + wide + 8 <= lx1;
+            const int C = lean ? wide : narrow;
+            const int xf = x - 8 < lx0 || x + C + 8 > lx1 ? MARCH_XFRAME : 0;
+            int well = 0;
+            for (int q = x; q < std::min(x + C, c->ntx) && !wcol.empty(); q++)
+                if (wcol[q] >= 0) well = MARCH_WELL;
+            if (lean) in.push_back(make_int4(x, C, bz, well));
+            else t.push_back(make_int4(x, C, bz, MARCH_FRAME | xf | well));
+            x += C;
+        }
+    }
+    *lean_tasks = in.size();
+    t.insert(t.end(), in.begin(), in.end());
+}
+
+// Columns per task: the widest chunks that still give every SM six lean tasks (wide chunks compute
+// fewer columns twice, but a warp by itself issues one instruction in six cycles); frame tasks
+// MARCH_NARROW.  Forward step, us, at 57 / 49 / 41 / 33 columns: 4001 x 1601 53.0 / 53.8 / 54.6 /
+// 57.7, 3301 x 1501 43.1 / - / 40.4 / 42.8, 3001 x 1403 38.5 / - / 35.7 / 34.1.
+static void march_tasks(const swd_ctx *c, std::vector<int4> &t, const std::vector<int> &wcol)
+{
+    for (int wide = 57; wide >= 33; wide -= 8) {
+        size_t n = 0;
+        t.clear();
+        march_tasks_of(c, t, wide, MARCH_NARROW, wcol, &n);
+        if (n >= (size_t)6 * std::max(c->nsm, 1)) return;
+    }
+}
+
+static MWave march_wave(swd_ctx *c, int k, int in_par)
+{
+    MWave w;
+    const int o = 1 - in_par;
+    w.p = fcopy(c, k, in_par, 0); w.vx = fcopy(c, k, in_par, 1); w.vz = fcopy(c, k, in_par, 2);
+    w.ppx = fcopy(c, k, in_par, 3); w.ppz = fcopy(c, k, in_par, 4);
+    w.po = fcopy(c, k, o, 0); w.vxo = fcopy(c, k, o, 1); w.vzo = fcopy(c, k, o, 2);
+    w.ppxo = fcopy(c, k, o, 3); w.ppzo = fcopy(c, k, o, 4);
+    w.pvx = F(c->wave[k][5]); w.pvz = F(c->wave[k][6]);
+    return w;
+}
+
+// One-wavefield forward pass by marches; a holds the plain kernels' arguments.  The final state
+// ends in wave[0].
+static int run_forward_march(swd_ctx *ctx, const FwdArgs &a, ShotPlan &P)
+{
+    CKR(zero_wave2(ctx, 0));
+    MFwdArgs m;
+    memset(&m, 0, sizeof m);
+    m.g = a.g; m.c = a.c; m.m = a.m; m.itp = a.itp; m.wav0 = a.wav0; m.sx = a.sx; m.sz = a.sz;
+    m.wells = a.wells; m.seis = a.seis; m.nt = a.nt;
+    std::vector<int4> tasks;
+    march_tasks(ctx, tasks, a.seis ? P.wcol : std::vector<int>());
+    CKR(ensure(ctx, ctx->marcht, sizeof(int4) * tasks.size()));
+    CK(cudaMemcpyAsync(ctx->marcht.p, tasks.data(), sizeof(int4) * tasks.size(), cudaMemcpyHostToDevice, ctx->stream));
+    m.task = (const int4 *)ctx->marcht.p;
+    // strips: FP32 straight into the store, 16-bit codes by way of an FP32 ring encoded once per
+    // captured chunk of steps
+    static_assert(MARCH_RING == GRAPH_K, "the ring holds one chunk of steps");
+    const dim3 grid = grid_blocks(ctx);
+    MEncodeArgs en;
+    memset(&en, 0, sizeof en);
+    int nlist = 0;
+    if (a.strips.buf && a.strips.prec == 0) {
+        m.strip = (float *)a.strips.buf;
+        m.slen = a.strips.slen;
+        m.ring = a.nt;
+    } else if (a.strips.buf) {
+        std::vector<int> list;
+        const int x1 = ctx->ntx - ctx->pmlc - 1, z1 = ctx->ntz - ctx->pmlc - 1, L = ctx->Lc, q = ctx->pmlc;
+        for (int by = 0; by < (int)grid.y; by++)
+            for (int bx = 0; bx < (int)grid.x; bx++) {
+                auto hit = [&](int xa, int xb, int za, int zb) { return by * 8 <= xb && by * 8 + 7 >= xa && bx * 128 <= zb && bx * 128 + 127 >= za; };
+                if (hit(q, x1, q, q + L - 1) || hit(q, x1, z1 - L + 1, z1) || hit(q, q + L - 1, q, z1) || hit(x1 - L + 1, x1, q, z1))
+                    list.push_back(by * grid.x + bx);
+            }
+        nlist = (int)list.size();
+        CKR(ensure(ctx, ctx->marchl, sizeof(int) * nlist));
+        CK(cudaMemcpyAsync(ctx->marchl.p, list.data(), sizeof(int) * nlist, cudaMemcpyHostToDevice, ctx->stream));
+        CKR(ensure(ctx, ctx->marchr, sizeof(float) * (size_t)MARCH_RING * a.strips.slen));
+        m.strip = F(ctx->marchr);
+        m.slen = a.strips.slen;
+        m.ring = MARCH_RING;
+        en.g = a.g; en.ringbuf = m.strip; en.itp = a.itp; en.strips = a.strips; en.list = I32(ctx->marchl); en.gx = grid.x;
+    }
+    m.w = march_wave(ctx, 0, 0);
+    const int nwarp = (int)tasks.size();
+    CK(cudaFuncSetAttribute(k_march_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, MARCH_FWD_SMEM));
+    auto launch = [&](int k, cudaEvent_t *) {
+        MFwdArgs b = m;
+        b.itoff = k;
+        b.w = march_wave(ctx, 0, k & 1);   // chunks start at even steps
+        k_march_fwd<<<nwarp, 32, MARCH_FWD_SMEM, ctx->stream>>>(b);
+        if (nlist && k == GRAPH_K - 1) k_march_encode<<<dim3(nlist, GRAPH_K), 128, 0, ctx->stream>>>(en);
+    };
+    struct { MFwdArgs m; MEncodeArgs e; int nlist, nwarp; } key;
+    memset(&key, 0, sizeof key);
+    key.m = m; key.e = en; key.nlist = nlist; key.nwarp = nwarp;
+    const int kid[1] = {0};
+    CKR(run_steps(ctx, ctx->gfwd, &key, sizeof key, 0, +1, a.nt, 1, kid, launch));
+    if (nlist && a.nt % GRAPH_K) {   // the steps after the last chunk
+        k_march_encode<<<dim3(nlist, a.nt % GRAPH_K), 128, 0, ctx->stream>>>(en);
+        CK(cudaGetLastError());
+    }
+    if (a.nt & 1)
+        for (int i = 0; i < 3; i++)
+            CK(cudaMemcpyAsync(ctx->wave[0][i].p, ctx->wave2[0][i].p, ctx->wave[0][i].n, cudaMemcpyDeviceToDevice, ctx->stream));
+    return SWD_OK;
 }
 
 static int run_forward_fused(swd_ctx *ctx, FwdJob &J, ShotPlan &P);
@@ -1334,6 +1470,7 @@ static int run_forward(swd_ctx *ctx, FwdJob &J, ShotPlan &P)
         CKR(run_resident(ctx, r, rp, 0, &ran));
         if (ran) return SWD_OK;
     }
+    if (nw == 1 && !a.ck.every && !a.ds.buf && !a.s0_out && !a.dkappa && !a.dck && march_ok(ctx)) return run_forward_march(ctx, a, P);
     // one wavefield without checkpoints: the velocity kernel with TMA-staged pressure
     // the plain single-wavefield forward (RTM forward, modelling without a twin): variants of the
     // velocity and pressure launches, chosen by the tuner when SWD_OPT_AUTOTUNE is on
