@@ -72,6 +72,7 @@ struct swd_ctx {
     // Born modelling and its adjoint: perturbation, gradient, background p-update sums,
     // context-owned checkpoints, adjoint scratch (Qx, Qz, Rx, Rz), adjoint source, aliases
     DevBuf dk, gk, s0, ckpt, adj[4], rbuf, alias;
+    DevBuf smo[3];           // smoothing: input, output, coefficients
     int ckpt_every = 50, ckpt_prec = SWD_STRIP_BF16;
     // batched RTM (swd_rtm_batch): every per-shot grid array is one allocation of per-shot slices
     struct BatchBufs {
@@ -148,6 +149,7 @@ struct swd_ctx {
                          &dk, &gk, &s0, &ckpt, &rbuf, &alias, &resll, &reserr, &marchl, &marcht, &marchr, &dpst, &dpsc, &cig, &cigring, &Ipart, &Spart, &Rpart};
         for (DevBuf *b : all) bufs.push_back(b);
         for (auto &b : adj) bufs.push_back(&b);
+        for (auto &b : smo) bufs.push_back(&b);
         for (auto &b : dcn) bufs.push_back(&b);
         DevBuf *ball[] = {&bat.dpdt, &bat.I, &bat.S, &bat.Ip, &bat.Sp, &bat.strips, &bat.scale, &bat.rdata, &bat.wcol, &bat.wmap,
                           &bat.desc, &bat.wav, &bat.reduce};
@@ -626,21 +628,26 @@ __global__ void k_stack_out(const double *__restrict__ st, float *out, int nx, i
 
 // Gaussian smoothing of ini_model_mine (acoustic_HLVSPRTMC.cpp:1514-1556): double
 // accumulation in the reference's loop order with unfused multiply and add, clamped
-// indices, rows iz < pml+8 unchanged.  Coefficients come from the host.
-__global__ void k_smooth(const float *__restrict__ vin, float *vout, const double *__restrict__ coef, int ntx, int ntz,
-                         int pml, int w)
+// indices, rows iz < pml+8 unchanged.  Coefficients come from the host.  The block's cells and
+// their window are converted to double once, in shared memory (8 + 2w columns of 32 + 2w rows):
+// converting at every tap kept the conversion unit busy (1669 x 869, 11 x 11 window: 120 -> 83 us).
+__global__ void __launch_bounds__(256) k_smooth(const float *__restrict__ vin, float *vout, const double *__restrict__ coef, int ntx,
+                                                int ntz, int pml, int w)
 {
-    const int iz = blockIdx.x * 32 + threadIdx.x + pml, ix = blockIdx.y * 8 + threadIdx.y + pml;
+    extern __shared__ double sv[];
+    const int z0 = blockIdx.x * 32 + pml, x0 = blockIdx.y * 8 + pml, nr = 32 + 2 * w, nc = 8 + 2 * w;
+    for (int c = threadIdx.y; c < nc; c += 8) {
+        const int x = min(max(x0 - w + c, 0), ntx - 1);
+        for (int r = threadIdx.x; r < nr; r += 32) sv[c * nr + r] = (double)vin[(size_t)x * ntz + min(max(z0 - w + r, 0), ntz - 1)];
+    }
+    __syncthreads();
+    const int iz = z0 + threadIdx.x, ix = x0 + threadIdx.y;
     if (iz > ntz - pml - 1 || ix > ntx - pml - 1) return;
     const int wx = 2 * w + 1;
+    const double *v = sv + threadIdx.y * nr + threadIdx.x;   // the window's first cell
     double s = 0.0;
-    for (int izw = iz - w; izw <= iz + w; izw++) {
-        const int iz1 = izw < 0 ? 0 : (izw > ntz - 1 ? ntz - 1 : izw);
-        for (int ixw = ix - w; ixw <= ix + w; ixw++) {
-            const int ix1 = ixw < 0 ? 0 : (ixw > ntx - 1 ? ntx - 1 : ixw);
-            s = __dadd_rn(s, __dmul_rn((double)vin[(size_t)ix1 * ntz + iz1], coef[(izw - iz + w) * wx + (ixw - ix + w)]));
-        }
-    }
+    for (int a = 0; a < wx; a++)
+        for (int b = 0; b < wx; b++) s = __dadd_rn(s, __dmul_rn(v[b * nr + a], __ldg(coef + a * wx + b)));
     const size_t ip = (size_t)ix * ntz + iz;
     vout[ip] = iz < pml + 8 ? vin[ip] : (float)s;
 }
@@ -698,20 +705,22 @@ __global__ void k_material_delta(const float *__restrict__ vp0, const float *__r
     }
 }
 
-// model_in_pml (acoustic_HLVSPRTMC.cpp:1428-1468): x-edges for interior rows, then z-edges
+// model_in_pml (acoustic_HLVSPRTMC.cpp:1428-1468): x-edges for interior rows, then z-edges; one
+// thread per frame cell
 __global__ void k_pml_x(float *v, int ntx, int ntz, int pml)
 {
-    const int iz = blockIdx.x * blockDim.x + threadIdx.x + pml;
+    const int iz = blockIdx.x * blockDim.x + threadIdx.x + pml, k = blockIdx.y;
     if (iz > ntz - pml - 1) return;
-    for (int ix = 0; ix <= pml - 1; ix++) v[(size_t)ix * ntz + iz] = v[(size_t)pml * ntz + iz];
-    for (int ix = ntx - pml; ix < ntx; ix++) v[(size_t)ix * ntz + iz] = v[(size_t)(ntx - pml - 1) * ntz + iz];
+    if (k < pml) v[(size_t)k * ntz + iz] = v[(size_t)pml * ntz + iz];
+    else v[(size_t)(ntx - 2 * pml + k) * ntz + iz] = v[(size_t)(ntx - pml - 1) * ntz + iz];
 }
 __global__ void k_pml_z(float *v, int ntx, int ntz, int pml)
 {
-    const int ix = blockIdx.x * blockDim.x + threadIdx.x;
+    const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+    const int ix = (int)(i / (2 * pml)), k = (int)(i % (2 * pml));
     if (ix >= ntx) return;
-    for (int iz = 0; iz <= pml - 1; iz++) v[(size_t)ix * ntz + iz] = v[(size_t)ix * ntz + pml];
-    for (int iz = ntz - pml; iz < ntz; iz++) v[(size_t)ix * ntz + iz] = v[(size_t)ix * ntz + (ntz - pml - 1)];
+    if (k < pml) v[(size_t)ix * ntz + k] = v[(size_t)ix * ntz + pml];
+    else v[(size_t)ix * ntz + ntz - 2 * pml + k] = v[(size_t)ix * ntz + (ntz - pml - 1)];
 }
 
 // ------------------------------------------------------------------------------------
@@ -2660,27 +2669,26 @@ int swd_smooth(swd_ctx *ctx, int ntx, int ntz, int pml, int window, float *vp)
         }
     for (auto &c : coef) c /= sum;
     const size_t n = (size_t)ntx * ntz;
-    DevBuf a, b, cf;
-    int rc = ensure(ctx, a, sizeof(float) * n);
-    if (rc == SWD_OK) rc = ensure(ctx, b, sizeof(float) * n);
-    if (rc == SWD_OK) rc = ensure(ctx, cf, sizeof(double) * coef.size());
-    if (rc == SWD_OK) rc = to_dev(ctx, a.p, vp, sizeof(float) * n);
-    if (rc == SWD_OK) {
-        cudaMemcpyAsync(cf.p, coef.data(), sizeof(double) * coef.size(), cudaMemcpyHostToDevice, ctx->stream);
-        cudaMemcpyAsync(b.p, a.p, sizeof(float) * n, cudaMemcpyDeviceToDevice, ctx->stream);
-        k_smooth<<<dim3((ntz - 2 * pml + 31) / 32, (ntx - 2 * pml + 7) / 8), dim3(32, 8), 0, ctx->stream>>>(
-            F(a), F(b), D(cf), ntx, ntz, pml, window);
-        k_pml_x<<<(ntz + 127) / 128, 128, 0, ctx->stream>>>(F(b), ntx, ntz, pml);
-        k_pml_z<<<(ntx + 127) / 128, 128, 0, ctx->stream>>>(F(b), ntx, ntz, pml);
-        cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) rc = fail(ctx, SWD_ERR_CUDA, "smoothing kernels: %s", cudaGetErrorString(e));
-        else rc = from_dev(ctx, vp, b.p, sizeof(float) * n);
+    // scratch kept by the context: three allocations and releases cost more than the smoothing
+    DevBuf &a = ctx->smo[0], &b = ctx->smo[1], &cf = ctx->smo[2];
+    CKR(ensure(ctx, a, sizeof(float) * n));
+    CKR(ensure(ctx, b, sizeof(float) * n));
+    CKR(ensure(ctx, cf, sizeof(double) * coef.size()));
+    CKR(to_dev(ctx, a.p, vp, sizeof(float) * n));
+    CK(cudaMemcpyAsync(cf.p, coef.data(), sizeof(double) * coef.size(), cudaMemcpyHostToDevice, ctx->stream));
+    CK(cudaMemcpyAsync(b.p, a.p, sizeof(float) * n, cudaMemcpyDeviceToDevice, ctx->stream));
+    const size_t sm = sizeof(double) * (8 + 2 * (size_t)window) * (32 + 2 * (size_t)window);
+    CK(cudaFuncSetAttribute(k_smooth, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    k_smooth<<<dim3((ntz - 2 * pml + 31) / 32, (ntx - 2 * pml + 7) / 8), dim3(32, 8), sm, ctx->stream>>>(
+        F(a), F(b), D(cf), ntx, ntz, pml, window);
+    if (pml > 0) {
+        k_pml_x<<<dim3((ntz - 2 * pml + 127) / 128, 2 * pml), 128, 0, ctx->stream>>>(F(b), ntx, ntz, pml);
+        k_pml_z<<<(unsigned)(((size_t)ntx * 2 * pml + 127) / 128), 128, 0, ctx->stream>>>(F(b), ntx, ntz, pml);
     }
-    cudaStreamSynchronize(ctx->stream);
-    cudaFree(a.p);
-    cudaFree(b.p);
-    cudaFree(cf.p);
-    return rc;
+    CK(cudaGetLastError());
+    CKR(from_dev(ctx, vp, b.p, sizeof(float) * n));
+    CK(cudaStreamSynchronize(ctx->stream));
+    return SWD_OK;
 }
 
 int swd_preprocess(swd_ctx *ctx, int r_n, int nt, float dt, const float *d, float *rms)
