@@ -222,6 +222,15 @@ __global__ void __launch_bounds__(256) k_adj_p(AdjArgs a)
     st4(a.qz + ip, Qz);
 }
 
+// Snapshot `snap` of the wavefield w into a checkpoint store, on the grid of k_fwd_v (whose CKPT
+// instantiation takes the same snapshots between steps).
+__global__ void __launch_bounds__(256) k_ckpt_save(Ckpt ck, Wave w, int snap, int ntx, int ntz, int ldz)
+{
+    int x, z0;
+    cell4(x, z0);
+    ckpt_save(ck, w, snap, x < ntx && z0 < ntz, (size_t)x * ldz + z0);
+}
+
 // Restore snapshot `snap` of a checkpoint store into the wavefield w; launched on the grid
 // of the saving kernel so the scale slots line up.
 __global__ void __launch_bounds__(256) k_ckpt_restore(Ckpt ck, Wave w, int snap, int ntx, int ntz, int ldz)

@@ -69,6 +69,21 @@ static FwdArgs born_fwd_args(swd_ctx *ctx, const swd_shot *s, bool twin)
 // steps [t0, t0+n) of the background field alone, S0 into slot it % s0_mod
 static int born_recompute(swd_ctx *ctx, const FwdArgs &base, int t0, int n, int klen)
 {
+    ResPlan rp;
+    if (klen >= RES_PIECE && resident_plan(ctx, 1, &rp)) {   // the whole segment in one launch
+        ResArgs r;
+        memset(&r, 0, sizeof r);
+        r.g = base.g; r.c = base.c; r.m = base.m;
+        r.w[0] = r.w[1] = base.w[0];
+        r.wav0 = base.wav0; r.wav1 = base.wav1;
+        r.sx = base.sx; r.sz = base.sz; r.nt = base.nt;
+        r.wells = base.wells;
+        r.s0 = base.s0_out; r.s0_stride = base.s0_stride; r.s0_mod = base.s0_mod;
+        r.t0 = t0; r.nsteps = n;
+        bool ran;
+        CKR(run_resident(ctx, r, rp, 3, &ran));
+        if (ran) return SWD_OK;
+    }
     const dim3 grid = grid_blocks(ctx);
     auto launch = [&](int k, cudaEvent_t *ev) {
         FwdArgs b = base;
@@ -137,8 +152,8 @@ static int check_ckpt(swd_ctx *ctx, const swd_shot *shot, const void *ckpt, size
     return SWD_OK;
 }
 
-int swd_born(swd_ctx *ctx, const swd_shot *shot, const float *rick, const float *dkappa, float *dseis, void *ckpt,
-             size_t ckpt_bytes)
+static int born_call(swd_ctx *ctx, const swd_shot *shot, const float *rick, const float *dkappa, float *dseis, void *ckpt,
+                     size_t ckpt_bytes)
 {
     CKR(check_ready(ctx));
     if (!rick || !dkappa || !dseis) return fail(ctx, SWD_ERR_ARG, "rick, dkappa and dseis are required");
@@ -165,8 +180,15 @@ int swd_born(swd_ctx *ctx, const swd_shot *shot, const float *rick, const float 
     return SWD_OK;
 }
 
-int swd_born_adjoint(swd_ctx *ctx, const swd_shot *shot, const float *rick, const float *resid, double *grad,
-                     const void *ckpt, size_t ckpt_bytes)
+int swd_born(swd_ctx *ctx, const swd_shot *shot, const float *rick, const float *dkappa, float *dseis, void *ckpt,
+             size_t ckpt_bytes)
+{
+    CKR(born_call(ctx, shot, rick, dkappa, dseis, ckpt, ckpt_bytes));
+    return resident_failed(ctx) ? born_call(ctx, shot, rick, dkappa, dseis, ckpt, ckpt_bytes) : SWD_OK;
+}
+
+static int born_adjoint_call(swd_ctx *ctx, const swd_shot *shot, const float *rick, const float *resid, double *grad,
+                             const void *ckpt, size_t ckpt_bytes)
 {
     CKR(check_ready(ctx));
     if (!rick || !resid || !grad) return fail(ctx, SWD_ERR_ARG, "rick, resid and grad are required");
@@ -258,6 +280,13 @@ int swd_born_adjoint(swd_ctx *ctx, const swd_shot *shot, const float *rick, cons
     CK(cudaStreamSynchronize(ctx->stream));
     prof_collect(ctx);
     return SWD_OK;
+}
+
+int swd_born_adjoint(swd_ctx *ctx, const swd_shot *shot, const float *rick, const float *resid, double *grad,
+                     const void *ckpt, size_t ckpt_bytes)
+{
+    CKR(born_adjoint_call(ctx, shot, rick, resid, grad, ckpt, ckpt_bytes));
+    return resident_failed(ctx) ? born_adjoint_call(ctx, shot, rick, resid, grad, ckpt, ckpt_bytes) : SWD_OK;
 }
 
 }  // extern "C"

@@ -52,8 +52,9 @@ __device__ __forceinline__ float4 mask4(float4 v, unsigned m)
     return make_float4(m & 1 ? v.x : 0.f, m & 2 ? v.y : 0.f, m & 4 ? v.z : 0.f, m & 8 ? v.w : 0.f);
 }
 
-// NW wavefields, XR columns per warp, at most MW warps, MODE 0 forward / 1 backward (wave 0 source, wave 1 receiver).
-// One CTA per SM.
+// NW wavefields, XR columns per warp, at most MW warps, MODE 0 forward / 1 backward (wave 0 source,
+// wave 1 receiver) / 2 Born (wave 0 background, wave 1 scattered field) / 3 background with its
+// p-update sums S0 written out.  One CTA per SM.
 //
 // Cells outside an update's guards get a zero coefficient instead of a branch (the field then
 // keeps its value), and the CPML terms are formed wherever the warp touches the frame (zero
@@ -164,6 +165,8 @@ __global__ void __launch_bounds__(32 * MW, 1) k_resident(const ResArgs a)
     // ---- own-cell arrays, one slot of TX columns each, in the order ck, cbx, cbz, then phi_p_x,
     // phi_p_z, phi_v_x, phi_v_z of each CPML wave, then the image sums and kap (backward)
     constexpr int NC = MODE == 1 ? 1 : NW, S_CK = 0, S_CBX = 1, S_CBZ = 2, S_PHI = 3, S_I = S_PHI + 4 * NC, S_S = S_I + 1, S_KAP = S_I + 2;
+    constexpr int S_DK = S_I;   // Born
+    constexpr bool BORN = MODE == 2, SUMS = MODE >= 2;
     float *slots = hzs + ((NW * 8 * TX + 2 * tabcap + 3) & ~3);
     auto keep = [&](int slot, const float *gp) {
 #pragma unroll
@@ -186,6 +189,7 @@ __global__ void __launch_bounds__(32 * MW, 1) k_resident(const ResArgs a)
         keep(S_S, a.Sp);
         keep(S_KAP, a.m.kap);
     }
+    if (BORN) keep(S_DK, a.dkappa);
     __syncthreads();
     const int nV = ntab[1], nP = ntab[0];
 
@@ -266,7 +270,7 @@ __global__ void __launch_bounds__(32 * MW, 1) k_resident(const ResArgs a)
 
 #pragma unroll 1
     for (int s = 0; s < a.nsteps; s++) {
-        const int it = MODE ? a.t0 - s : a.t0 + s;
+        const int it = MODE == 1 ? a.t0 - s : a.t0 + s;
         const unsigned tag = a.epoch + 1u + (unsigned)s;
         // the thread's addresses are formed anew in every step (opaque copies), so that the compiler
         // does not keep dozens of loop invariants in registers and spill the fields for them
@@ -376,7 +380,7 @@ __global__ void __launch_bounds__(32 * MW, 1) k_resident(const ResArgs a)
         xpb = xp + co;
         zpb = zp + 4 * lo;
         Sb = slots + co * TZ + 4 * lo;
-        float4 dp[MODE == 1 ? XR : 1];   // backward: the source's p-update sum of interior cells
+        float4 dp[MODE == 0 ? 1 : XR];   // backward: the source's p-update sum of interior cells; Born: field 0's of updated cells
 #pragma unroll
         for (int k = 0; k < NW; k++) {
             const bool src = MODE == 1 && k == 0;
@@ -450,10 +454,22 @@ __global__ void __launch_bounds__(32 * MW, 1) k_resident(const ResArgs a)
                         for (int q = 0; q < 4; q++) el(f, q) = elc(az, q) != 0.f ? elc(bzv, q) * elc(f, q) + elc(az, q) * elc(e, q) : 0.f;
                         st4(Sb + (phi + 3) * ss + i * TZ, f);
                     }
-                    if (mk) kc = mask4(kc, (x >= LC && x <= ntx - LC) ? mp : 0u);
+                    const unsigned gp = mk ? ((x >= LC && x <= ntx - LC) ? mp : 0u) : 15u;
+                    if (mk) kc = mask4(kc, gp);
+                    if (SUMS && k == 0) {
+#pragma unroll
+                        for (int q = 0; q < 4; q++) el(dp[i], q) = elc(d, q) + elc(e, q) + elc(f, q);
+                        if (mk) dp[i] = mask4(dp[i], gp);
+                        if (MODE == 3 && has(i)) st4(a.s0 + (size_t)(it % a.s0_mod) * a.s0_stride + cell(i), dp[i]);
+                    }
 #pragma unroll
                     for (int q = 0; q < 4; q++) el(p, q) = elc(kc, q) * (elc(d, q) + elc(e, q) + elc(f, q)) + elc(p, q);
-                    if (MODE == 0 && sx_here && x == a.sx) {
+                    if (BORN && k == 1) {   // secondary source of the scattered field
+                        const float4 dk = own(S_DK, i);
+#pragma unroll
+                        for (int q = 0; q < 4; q++) el(p, q) += g.dt * elc(dk, q) * elc(dp[i], q);
+                    }
+                    if (MODE != 1 && sx_here && x == a.sx) {
 #pragma unroll
                         for (int q = 0; q < 4; q++)
                             if (a.sz == z0 + q) el(p, q) += (k == 0 ? a.wav0[it] : a.wav1[it]);
@@ -538,13 +554,13 @@ __global__ void __launch_bounds__(32 * MW, 1) k_resident(const ResArgs a)
                 for (int i = 0; i < XR; i++) ll_send4(ll + aZ + k * astep + 2 * i, ld4(Pk + i * PZ), tag);
             }
         }
-        if (MODE == 0) {   // records and strips, nobody waits for them
+        if (MODE != 1) {   // records (Born: of the scattered field) and strips, nobody waits for them
             if (wi >= 0 && in) {
 #pragma unroll
                 for (int i = 0; i < XR; i++) {
                     const int wc = wcs[co + i];
                     if (wc < 0 || !a.seis) continue;
-                    const float4 p = ld4(Pb + i * PZ);
+                    const float4 p = ld4(Pb + (BORN ? psz : 0) + i * PZ);
                     int4 tr = wtr;
                     if (i != wi) tr = __ldg(reinterpret_cast<const int4 *>(a.wells.wmap + (size_t)wc * ldz + z0));
 #pragma unroll
@@ -597,10 +613,17 @@ __global__ void __launch_bounds__(32 * MW, 1) k_resident(const ResArgs a)
                 st4(a.w[k].p + cell(i), ld4(P(k, c0 + i, 4 * lane)));
                 st4(a.w[k].vx + cell(i), ld4(V(k, c0 + i, 4 * lane)));
                 st4(a.w[k].vz + cell(i), vz[k][i]);
+                if (SUMS) {   // a piece of a pass: the CPML memories go on in the next one
+                    const float *q = slots + (S_PHI + 4 * k) * TX * TZ + (c0 + i) * TZ + 4 * lane;
+                    st4(a.w[k].ppx + cell(i), ld4(q));
+                    st4(a.w[k].ppz + cell(i), ld4(q + TX * TZ));
+                    st4(a.w[k].pvx + cell(i), ld4(q + 2 * TX * TZ));
+                    st4(a.w[k].pvz + cell(i), ld4(q + 3 * TX * TZ));
+                }
             }
 }
 
-bool res_plan(int ntx, int ntz, int nsm, size_t smem_max, int nw, ResPlan *p)
+bool res_plan(int ntx, int ntz, int nsm, size_t smem_max, int nw, bool born, ResPlan *p)
 {
     if (ntx < 48 || ntz < 48) return false;   // the strip bands of both sides never meet in a thread's rows
     p->nw = nw;
@@ -613,7 +636,7 @@ bool res_plan(int ntx, int ntz, int nsm, size_t smem_max, int nw, ResPlan *p)
     if (p->XR == 2 && p->nwarps > RES_MAXW2) return false;
     p->TX = p->XR * p->nwarps;
     p->GX = (ntx + p->TX - 1) / p->TX;
-    p->smem = res_smem(p->TX, nw);
+    p->smem = res_smem(p->TX, nw) + (born ? sizeof(float) * p->TX * RES_TZ : 0);
     p->ll_bytes = sizeof(ulonglong2) * (size_t)p->GX * p->GZ * nw * 2 * res_pieces(p->TX);
     return p->smem + 1024 <= smem_max;   // 1 KB: static shared memory
 }
@@ -638,6 +661,8 @@ static cudaError_t launch_xr(const ResArgs &a, const ResPlan &p, cudaStream_t st
 cudaError_t res_launch(const ResArgs &a, const ResPlan &p, int mode, cudaStream_t st)
 {
     if (mode == 1) return launch_xr<2, 1>(a, p, st);
+    if (mode == 2) return launch_xr<2, 2>(a, p, st);
+    if (mode == 3) return launch_xr<1, 3>(a, p, st);
     return p.nw == 2 ? launch_xr<2, 0>(a, p, st) : launch_xr<1, 0>(a, p, st);
 }
 

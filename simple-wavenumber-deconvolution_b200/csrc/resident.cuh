@@ -13,7 +13,8 @@
 //
 // Measured per time step (B200, 30-cell frame): RTM, forward plus backward, 401 x 201 18.2 -> 9.7
 // us, 801 x 401 20.0 -> 14.1 us, 100 x 60 17.0 -> 8.4 us; modelling with the Hilbert twin
-// 401 x 201 10.3 -> 5.3 us, 801 x 401 11.1 -> 7.8 us.
+// 401 x 201 10.3 -> 5.3 us, 801 x 401 11.1 -> 7.8 us; Born modelling with checkpoints every 64 steps
+// 401 x 201 10.3 -> 5.5 us, 801 x 401 10.8 -> 8.0 us.
 //
 // A warp owns XR adjacent columns of the tile, a lane four rows of them, as in the plain kernels;
 // the x taps come from a register window over the neighbouring columns.  One column per warp up to
@@ -45,6 +46,11 @@ constexpr int RES_PZ = RES_TZ + 8;   // pressure column in shared memory with it
 constexpr int RES_MAXW1 = 16;        // warps of a CTA at most, one column per warp
 constexpr int RES_MAXW2 = 12;        // two columns per warp; one column with the larger register budget
 constexpr int RES_SPIN = 1 << 22;
+// Steps of a piece at least: Born passes stop at every checkpoint, and a launch that loads and
+// stores the whole state costs about 15 to 25 us.  Born plus adjoint pass per step with checkpoints
+// every 4 / 8 / 64 steps: 401 x 201 31.2 -> 27.1 / 27.8 -> 21.8 / 24.9 -> 17.4 us, 801 x 401
+// 32.5 -> 33.5 / 28.9 -> 27.3 / 26.2 -> 22.2 us.
+constexpr int RES_PIECE = 8;
 
 // Tiling of a grid: CTAs GX x GZ, TX = XR * nwarps columns per tile.
 struct ResPlan {
@@ -67,6 +73,10 @@ struct ResArgs {
     const float *rdata;    // backward: injected data
     double *I, *S;
     float *Ip, *Sp;
+    const float *dkappa;   // Born: bulk-modulus perturbation
+    float *s0;             // p-update sums, slot it % s0_mod
+    long long s0_stride;
+    int s0_mod;
     int t0, nsteps;        // steps t0, t0 + 1, ... (forward) or t0, t0 - 1, ... (backward)
     int TX, GX, GZ;
     uint4 *ll;             // exchange words
@@ -88,10 +98,11 @@ __host__ __device__ inline size_t res_smem(int TX, int nw)
                             (size_t)nw * (8 * TX + 2 * (448 + 4 * TX)) + (size_t)(nw == 1 ? 7 : 11) * TX * RES_TZ);
 }
 
-// launches nsteps steps; MODE 0 forward, 1 backward (plan.nw == 2)
+// launches nsteps steps; mode 0 forward, 1 backward (plan.nw == 2), 2 Born (plan.nw == 2), 3 forward
+// with S0 (plan.nw == 1); modes 2 and 3 may run a pass in pieces
 cudaError_t res_launch(const ResArgs &a, const ResPlan &p, int mode, cudaStream_t st);
 // tiling of an ntx x ntz grid on nsm SMs with smem_max bytes of shared memory per CTA; false
-// when the wavefields do not fit
-bool res_plan(int ntx, int ntz, int nsm, size_t smem_max, int nw, ResPlan *p);
+// when the wavefields do not fit; born: with the perturbation of mode 2
+bool res_plan(int ntx, int ntz, int nsm, size_t smem_max, int nw, bool born, ResPlan *p);
 
 }  // namespace swd

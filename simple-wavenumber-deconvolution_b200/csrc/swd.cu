@@ -1194,10 +1194,10 @@ static bool default_steps(const swd_ctx *c)
 // wavefields fit on the chip; plan receives the tiling for nw wavefields.  The plain kernels keep
 // every other case: larger grids, other stencil lengths, 16-bit strips, profiling, the kernel
 // variants the options select.
-static bool resident_plan(const swd_ctx *c, int nw, ResPlan *plan)
+static bool resident_plan(const swd_ctx *c, int nw, ResPlan *plan, bool born = false)
 {
     if (!c->use_resident || !c->coop || c->Lc != RES_LC || !c->use_graphs || !default_steps(c)) return false;
-    return res_plan(c->ntx, c->ntz, c->nsm, c->smem_max, nw, plan);
+    return res_plan(c->ntx, c->ntz, c->nsm, c->smem_max, nw, born, plan);
 }
 
 // Two of these launches must not share the device (each would hold SMs the other waits for), so
@@ -1462,10 +1462,39 @@ static int run_forward(swd_ctx *ctx, FwdJob &J, ShotPlan &P)
     a.wav0 = F(ctx->wav);
     a.wav1 = J.twin ? F(ctx->wav) + nt : F(ctx->wav);
     const int nw = J.twin ? 2 : 1;
-    // one field, or a field and its twin, whose grid fits on the chip: the whole pass in one launch
     ResPlan rp;
-    if (!a.ck.every && !a.ds.buf && !a.s0_out && !a.dkappa && !a.dck && (!a.strips.buf || a.strips.prec == 0) &&
-        resident_plan(ctx, nw, &rp)) {
+    // Born modelling on the chip, in pieces of the checkpoint interval (RES_PIECE)
+    if (a.dkappa && nw == 2 && !a.s0_out && !a.ds.buf && !a.strips.buf && (!a.ck.every || a.ck.every >= RES_PIECE) &&
+        resident_plan(ctx, 2, &rp, true)) {
+        ResArgs r;
+        memset(&r, 0, sizeof r);
+        r.g = a.g; r.c = a.c; r.m = a.m;
+        r.w[0] = a.w[0]; r.w[1] = a.w[1];
+        r.wav0 = a.wav0; r.wav1 = a.wav1;
+        r.sx = a.sx; r.sz = a.sz; r.nt = nt;
+        r.wells = a.wells; r.seis = a.seis; r.dkappa = a.dkappa;
+        const int piece = a.ck.every > 0 ? a.ck.every : nt;
+        bool ran = true;
+        for (int t0 = 0; t0 < nt && ran; t0 += piece) {
+            if (a.ck.every > 0) {
+                k_ckpt_save<<<grid, dim3(32, 8), 0, ctx->stream>>>(a.ck, a.w[0], t0 / piece, ctx->ntx, ctx->ntz, ctx->ldz);
+                ctx->launches++;
+            }
+            r.t0 = t0;
+            r.nsteps = std::min(piece, nt - t0);
+            CKR(run_resident(ctx, r, rp, 2, &ran));
+        }
+        if (ran) {
+            CK(cudaGetLastError());
+            return SWD_OK;
+        }
+        CKR(zero_wave(ctx, 0));   // a refused launch: from the start with the step kernels
+        CKR(zero_wave(ctx, 1));
+    }
+    // one field (and its p-update sums), or a field and its twin, whose grid fits on the chip: the
+    // whole pass in one launch
+    if (!a.ck.every && !a.ds.buf && !a.dkappa && !a.dck && (!a.strips.buf || a.strips.prec == 0) &&
+        (!a.s0_out || (nw == 1 && !a.strips.buf)) && resident_plan(ctx, nw, &rp)) {
         ResArgs r;
         memset(&r, 0, sizeof r);
         r.g = a.g; r.c = a.c; r.m = a.m;
@@ -1474,9 +1503,10 @@ static int run_forward(swd_ctx *ctx, FwdJob &J, ShotPlan &P)
         r.sx = a.sx; r.sz = a.sz; r.nt = nt;
         r.wells = a.wells; r.seis = a.seis; r.colmap = a.colmap; r.colbuf = a.colbuf;
         r.strips = a.strips;
+        r.s0 = a.s0_out; r.s0_stride = a.s0_stride; r.s0_mod = a.s0_mod;
         r.t0 = 0; r.nsteps = nt;
         bool ran;
-        CKR(run_resident(ctx, r, rp, 0, &ran));
+        CKR(run_resident(ctx, r, rp, a.s0_out ? 3 : 0, &ran));
         if (ran) return SWD_OK;
     }
     if (nw == 1 && !a.ck.every && !a.ds.buf && !a.s0_out && !a.dkappa && !a.dck && march_ok(ctx)) return run_forward_march(ctx, a, P);

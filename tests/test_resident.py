@@ -7,6 +7,7 @@ warp and per cell column, duplicates, frame cells), the source inside the strip 
 frame.  The arithmetic is the same term by term, so the comparison is exact."""
 import numpy as np
 import pytest
+import torch
 
 pytestmark = pytest.mark.gpu
 
@@ -81,3 +82,39 @@ def test_resident_needs_its_sizes(swd):
         n0 = E.launch_count()
         E.rtm_forward(s, swd.ricker_wave(nt, 25.0, 5e-4))
         assert E.launch_count() - n0 >= 2 * nt
+
+
+@pytest.mark.parametrize("name", list(GRIDS))
+def test_resident_born_same_bits(swd, name):
+    """Born modelling and the recomputed background of its adjoint, in pieces of the checkpoint
+    interval: full storage, the shortest piece taken, a last piece of one step, one piece only, and
+    an interval below the shortest piece; checkpoints of 32 and of 16 bits."""
+    nx, nz, pml = GRIDS[name]
+    nt = 121
+    E, rng, (ntx, ntz) = _engine(swd, nx, nz, pml, nt, 7)
+    pmlc = pml + 4
+    n = 40
+    rix, riz = rng.integers(0, ntx, n).astype(np.int32), rng.integers(0, ntz, n).astype(np.int32)
+    rix[:20] = pmlc + nx // 2
+    riz[:20] = np.minimum(pmlc + np.arange(20), ntz - 1)
+    riz[1] = riz[0]
+    rick = swd.ricker_wave(nt, 25.0, 5e-4)
+    s = swd.ShotSpec(pmlc + nx // 2, pmlc + 1, rix, riz, nt)
+    dk = (rng.standard_normal((ntx, ntz)) * 1e7).astype(np.float32)
+    resid = rng.standard_normal((n, nt)).astype(np.float32)
+    out = {}
+    for res in (0, 1):
+        E.set_option(swd.OPT_RESIDENT, res)
+        r = []
+        for every, prec in ((0, swd.STRIP_F32), (8, swd.STRIP_F32), (40, swd.STRIP_BF16), (500, swd.STRIP_I16), (7, swd.STRIP_F16)):
+            E.set_checkpointing(every, prec)
+            ck = torch.empty(max(16, E.checkpoint_bytes(nt)), dtype=torch.uint8, device="cuda") if every else None
+            n0 = E.launch_count()
+            r.append(E.born(s, rick, dk, ckpt=ck))
+            assert E.launch_count() - n0 >= 2 * nt if not res or 0 < every < 8 else E.launch_count() - n0 < nt
+            r += [E.born_adjoint(s, rick, resid, ckpt=ck), E.born_adjoint(s, rick, resid)]
+        out[res] = r
+    assert E.get_option(swd.OPT_RESIDENT) == 1
+    for i, (a, b) in enumerate(zip(out[1], out[0])):
+        assert np.abs(b).max() > 0, i
+        assert np.array_equal(a, b), i
