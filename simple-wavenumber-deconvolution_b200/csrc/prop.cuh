@@ -70,7 +70,7 @@ struct DpStore {
 };
 
 // forward pressure-kernel modes
-constexpr int FP_PLAIN = 0, FP_BORN = 1, FP_STORE = 2, FP_SCAT = 3;
+constexpr int FP_PLAIN = 0, FP_BORN = 1, FP_STORE = 2, FP_SCAT = 3, FP_SCAT_SEG = 4;
 
 // One wavefield updated in place.
 struct Wave {
@@ -538,9 +538,19 @@ struct FwdArgs {
     // dcb * (d + phi) of field 0 in the velocity updates and dck * S0 in the pressure update
     // (dcb, dck: coefficient differences m1 - m, formed in double).  The receivers record field
     // 1; colcomp >= 0 writes field 1's column into that component of colbuf only.
+    //
+    // dseg, one byte per column and 128 rows (a warp's cells): bit 0 where the velocity
+    // coefficients of the models differ, bit 1 where the pressure coefficients do.  Elsewhere
+    // m1 is m and the differences are zero, and both fields use m: a pass that streams from HBM
+    // reads 21 arrays a step instead of 27 where the scatterers are isolated (4001 x 1601,
+    // scatterers every 19 cells: 146 -> 120 us per step, of which 10 by the reads ahead; 2001 x 1001
+    // 56 -> 43, 1601 x 801 33 -> 28).  nullptr where more than half of the bytes are set (the
+    // question costs a dense difference 3%: 2001 x 1001 56.0 -> 57.5 us).
     Mat m1;
     const float *dcbx, *dcbz, *dck;
+    const unsigned char *dseg;
     int colcomp;
+    int ahead;           // host: launch the AHEAD instantiations (ahead_cell) where there are any
 };
 
 // The shot's view of a batched forward launch; false when the shot's record has ended.
@@ -638,13 +648,34 @@ __device__ __forceinline__ void cell4(int &x, int &z0)
     x = blockIdx.y * 8 + threadIdx.y;
 }
 
+// Operands of a later column into L2 at the start of a step kernel.  A step that streams from HBM is
+// bound by the DRAM latency of each warp's few loads in flight (4.4 TB/s; registers for more loads
+// would cost resident warps); a prefetch holds no register and nothing waits for it, so the block
+// AHEAD_COLS on finds its lines in L2.  Us per step, without / with: RTM backward 4001 x 1601
+// 131.8 / 116.4, 2501 x 1203 66.8 / 63.7, 2001 x 1001 44.8 / 44.4, 1601 x 801 26.3 / 27.7; scattered
+// field 4001 x 1601 150.8 / 130.1, 1601 x 801 31.6 / 32.5; field and twin 4001 x 1601 127.7 / 106.4.
+// 24 to 64 columns ahead give the same, 1 column ahead half of it, from 320 on lines are evicted
+// again before they are read.  Its own instantiations (stencil order 4): as a branch it cost the grids
+// that stay in L2 3% in registers.
+constexpr int AHEAD_COLS = 40;
+__device__ __forceinline__ size_t ahead_cell(const Geo &g, int x, int z0)
+{
+    return (size_t)min(x + AHEAD_COLS, g.ntx - 1) * g.ldz + z0;
+}
+__device__ __forceinline__ void prefetch_wave(const Wave &w, size_t ip)
+{
+    prefetch_l2(w.p + ip);
+    prefetch_l2(w.vx + ip);
+    prefetch_l2(w.vz + ip);
+}
+
 // MB > 0 bounds the registers to MB blocks of 256 per SM (the variant for passes whose working
 // set streams from HBM, where more resident warps keep more bytes in flight; same bits).  The
 // twins without checkpoints are bounded to 5 blocks: the plain twin 48 registers instead of 52
 // (AFor's velocity step 12.5 -> 11.6 us on 1601x801), the scattered-field twin 48 instead of 54
 // (90.5 -> 80.6 us on 4001x1601).  The batched kernel, whose batch streams from HBM, takes 6
 // (40 registers, no spill: 27.5 -> 24.3 us per step of four 1601x801 shots).
-template <int LC, int NW, bool CKPT, bool BATCH = false, bool SCAT = false, int MB = 0>
+template <int LC, int NW, bool CKPT, bool BATCH = false, int SCAT = 0, int MB = 0, bool AHEAD = false>
 __global__ void __launch_bounds__(256, MB > 0 ? MB : ((NW == 2 && LC <= 4 && !CKPT) ? 5 : (BATCH && LC <= 4) ? 6 : 0))
     k_fwd_v(const FwdArgs a0)
 {
@@ -661,18 +692,32 @@ __global__ void __launch_bounds__(256, MB > 0 ? MB : ((NW == 2 && LC <= 4 && !CK
             ckpt_save(a.ck, a.w[0], it / a.ck.every, x < a.g.ntx && z0 < a.g.ntz, (size_t)x * a.g.ldz + z0);
     }
     if (x >= a.g.ntx || z0 >= a.g.ntz) return;
-    if constexpr (SCAT) {
+    if constexpr (AHEAD) {
+        const size_t ip = ahead_cell(a.g, x, z0);
+#pragma unroll
+        for (int k = 0; k < NW; k++) prefetch_wave(a.w[k], ip);
+        prefetch_l2(a.m.cbx + ip);
+        prefetch_l2(a.m.cbz + ip);
+    }
+    if constexpr (SCAT != 0) {   // 1: the models differ everywhere, 2: where dseg says so
         static_assert(NW == 2, "the scattered field runs beside its background");
         float4 sx, sz;
         const PGlobal p0{a.w[0].p, a.g.ldz}, p1{a.w[1].p, a.g.ldz};
+        const bool diff = SCAT == 1 || (__ldg(a.dseg + (size_t)x * gridDim.x + blockIdx.x) & 1);
         if (lean_block(a.g)) {
             v_update4_l<LC, false, PGlobal, 1, true>(a.g, a.c, a.m, a.w[0], x, z0, p0, &sx, &sz);
-            v_update4_l<LC, false, PGlobal, 2, true>(a.g, a.c, a.m1, a.w[1], x, z0, p1, &sx, &sz, a.dcbx,
-                                                     a.dcbz);
+            if (diff)
+                v_update4_l<LC, false, PGlobal, 2, true>(a.g, a.c, a.m1, a.w[1], x, z0, p1, &sx, &sz, a.dcbx,
+                                                         a.dcbz);
+            else
+                v_update4_l<LC, false, PGlobal, 0, true>(a.g, a.c, a.m, a.w[1], x, z0, p1);
         } else {
             v_update4_l<LC, false, PGlobal, 1>(a.g, a.c, a.m, a.w[0], x, z0, p0, &sx, &sz);
-            v_update4_l<LC, false, PGlobal, 2>(a.g, a.c, a.m1, a.w[1], x, z0, p1, &sx, &sz, a.dcbx,
-                                               a.dcbz);
+            if (diff)
+                v_update4_l<LC, false, PGlobal, 2>(a.g, a.c, a.m1, a.w[1], x, z0, p1, &sx, &sz, a.dcbx,
+                                                   a.dcbz);
+            else
+                v_update4_l<LC, false, PGlobal, 0>(a.g, a.c, a.m, a.w[1], x, z0, p1);
         }
     } else if (lean_block(a.g)) {
 #pragma unroll
@@ -704,17 +749,17 @@ constexpr int fwd_p_min_blocks()
     if (NW == 1) return MODE == FP_BORN ? 1 : 5;
     // Born twin: 4 (64 registers, no spill); the scattered-field twin at 5 (48 registers, a
     // 108-byte spill) ran 72.5 -> 68.9 us per step on 4001x1601, ahead of 4 blocks
-    return (MODE == FP_PLAIN || MODE == FP_SCAT) ? 5 : 4;
+    return (MODE == FP_PLAIN || MODE == FP_SCAT || MODE == FP_SCAT_SEG) ? 5 : 4;
 }
 
 // MB > 0 asks the register allocator for MB blocks of 256 per SM instead of the default bound
 // (the autotuner's register-bound variants of the plain kernel; same code, same bits)
-template <int LC, int NW, int MODE, bool BATCH = false, int MB = 0>
+template <int LC, int NW, int MODE, bool BATCH = false, int MB = 0, bool AHEAD = false>
 __global__ void __launch_bounds__(256, (MB > 0 ? MB : fwd_p_min_blocks<LC, NW, MODE, BATCH>()))
     k_fwd_p(const FwdArgs a0)
 {
     pdl_begin();
-    constexpr bool BORN = MODE == FP_BORN, SCAT = MODE == FP_SCAT;
+    constexpr bool BORN = MODE == FP_BORN, SEG = MODE == FP_SCAT_SEG, SCAT = MODE == FP_SCAT || SEG;
     FwdArgs a = a0;
     const int it = *a.itp + a.itoff;
     if constexpr (BATCH) {
@@ -731,16 +776,24 @@ __global__ void __launch_bounds__(256, (MB > 0 ? MB : fwd_p_min_blocks<LC, NW, M
     float4 s0 = make_float4(0.f, 0.f, 0.f, 0.f);   // field 0's p-update sum (Born, store)
     if (in) {
         const size_t ip = (size_t)x * g.ldz + z0;
+        if constexpr (AHEAD) {
+            const size_t ia = ahead_cell(g, x, z0);
+#pragma unroll
+            for (int k = 0; k < NW; k++) prefetch_wave(a.w[k], ia);
+            prefetch_l2(a.m.ck + ia);
+        }
+        bool diff = SCAT;   // whether the models differ in this warp's cells
+        if constexpr (SEG) diff = __ldg(a.dseg + (size_t)x * gridDim.x + blockIdx.x) & 2;
 #pragma unroll
         for (int w = 0; w < NW; w++) {
             bool upd[4];
-            const Mat &mw = (SCAT && w == 1) ? a.m1 : a.m;
+            const Mat &mw = (SCAT && w == 1 && diff) ? a.m1 : a.m;
             float4 *ss = (MODE != FP_PLAIN && w == 0) ? &s0 : nullptr;
             if (lean) p_update4<LC, false, true>(g, a.c, mw, a.w[w], x, z0, pn[w], upd, ss);
             else p_update4<LC>(g, a.c, mw, a.w[w], x, z0, pn[w], upd, ss);
             bool any = upd[0] || upd[1] || upd[2] || upd[3];
             if constexpr (SCAT) {
-                if (w == 1) {
+                if (w == 1 && diff) {
                     const float4 dk = ldg4(a.dck + ip);
 #pragma unroll
                     for (int k = 0; k < 4; k++)
@@ -842,6 +895,7 @@ struct BwdArgs {
     float *Ip, *Sp, *Rp; // FP32 sums of the current block of IMG_BLOCK steps (nullptr: FP64 every step)
     Batch bt;            // the BATCH instantiations: shot = blockIdx.z
     DpStore ds;          // stored-source backward (k_bwd_rcv_*): dp/dt of forward step it+1
+    int ahead;           // as in FwdArgs
 };
 
 // The shot's view of a batched backward launch: its own time index (every shot of a batch
@@ -1150,7 +1204,7 @@ __global__ void __launch_bounds__(256, (LC <= 4 && !BATCH) ? 5 : 1) k_bwd_2(cons
 // them after every step, use k_bwd_1 + k_bwd_2.
 // ------------------------------------------------------------------------------------
 // MB as in k_fwd_v
-template <int LC, bool BATCH = false, int MB = 0>
+template <int LC, bool BATCH = false, int MB = 0, bool AHEAD = false>
 __global__ void __launch_bounds__(256, MB) k_bwd_v(const BwdArgs a0)
 {
     pdl_begin();
@@ -1164,6 +1218,13 @@ __global__ void __launch_bounds__(256, MB) k_bwd_v(const BwdArgs a0)
     const Geo &g = a.g;
     if (x >= g.ntx || z0 >= g.ntz) return;
     const size_t ip = (size_t)x * g.ldz + z0;
+    if constexpr (AHEAD) {
+        const size_t ia = ahead_cell(g, x, z0);
+        prefetch_wave(a.s, ia);
+        prefetch_wave(a.r, ia);
+        prefetch_l2(a.m.cbx + ia);
+        prefetch_l2(a.m.cbz + ia);
+    }
     if (lean_block(g)) {   // every cell interior, no CPML term, no strip
         const bool in[4] = {true, true, true, true};
         if (it < a.nt - 2) src_v_phase<LC>(a, x, z0, ip, in);
@@ -1176,7 +1237,7 @@ __global__ void __launch_bounds__(256, MB) k_bwd_v(const BwdArgs a0)
     v_update4<LC, true>(g, a.c, a.m, a.r, x, z0);
 }
 
-template <int LC, bool BATCH = false, int MB = 0>
+template <int LC, bool BATCH = false, int MB = 0, bool AHEAD = false>
 __global__ void __launch_bounds__(256, MB > 0 ? MB : (LC > 4 ? 1 : BATCH ? BATCH_BWD_P_MIN_BLOCKS : 5)) k_bwd_p(const BwdArgs a0)
 {
     pdl_begin();
@@ -1190,9 +1251,17 @@ __global__ void __launch_bounds__(256, MB > 0 ? MB : (LC > 4 ? 1 : BATCH ? BATCH
     const Geo &g = a.g;
     if (x >= g.ntx || z0 >= g.ntz) return;
     const size_t ip = (size_t)x * g.ldz + z0;
+    if constexpr (AHEAD) {
+        const size_t ia = ahead_cell(g, x, z0);
+        prefetch_wave(a.s, ia);
+        prefetch_wave(a.r, ia);
+        prefetch_l2(a.m.ck + ia);
+        prefetch_l2(a.m.kap + ia);
+        image_prefetch(a, ia, it);
+    }
     if (lean_block(g)) {   // every cell interior, no CPML term, no strip
         const bool in[4] = {true, true, true, true};
-        image_prefetch(a, ip, it);
+        if (!AHEAD) image_prefetch(a, ip, it);
         float4 dp;
         src_p_phase<LC, true>(a, it, x, z0, ip, in, true, dp);
         const float4 pr = rcv_p_phase<LC, true>(a, it, x, z0, ip);
@@ -1201,7 +1270,7 @@ __global__ void __launch_bounds__(256, MB > 0 ? MB : (LC > 4 ? 1 : BATCH ? BATCH
     }
     bool in[4];
     const bool any = interior4(g, x, z0, in);
-    if (any) image_prefetch(a, ip, it);
+    if (any && !AHEAD) image_prefetch(a, ip, it);
     float4 dp;
     src_p_phase<LC>(a, it, x, z0, ip, in, any, dp);
     const float4 pr = rcv_p_phase<LC>(a, it, x, z0, ip);

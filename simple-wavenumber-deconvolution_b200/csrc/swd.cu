@@ -54,8 +54,8 @@ struct swd_ctx {
     DevBuf vp, rho, cpml[8], mat[4];
     // perturbed model of the exact scattered field (swd_set_scatter_model): its coefficients
     // and the coefficient differences dcbx, dcbz, dck against the background
-    DevBuf vp1, rho1, mat1[4], dmat[3];
-    bool have_scatter = false;
+    DevBuf vp1, rho1, mat1[4], dmat[3], dseg;
+    bool have_scatter = false, scatter_dense = false;   // dense: the models differ in most places
     // wavefields: w[0], w[1] (7 arrays each), dp/dt
     DevBuf wave[2][7], dpdt;
     // second copies of p, vx, vz, phi_p_x, phi_p_z for the fused (double-buffered) path
@@ -160,6 +160,7 @@ struct swd_ctx {
         for (auto &b : mat) bufs.push_back(&b);
         for (auto &b : mat1) bufs.push_back(&b);
         for (auto &b : dmat) bufs.push_back(&b);
+        bufs.push_back(&dseg);
         bufs.push_back(&vp1);
         bufs.push_back(&rho1);
         for (auto &w : wave)
@@ -697,12 +698,33 @@ __global__ void k_material_delta(const float *__restrict__ vp0, const float *__r
             const double v0 = vp0[i], v1 = vp1[i], r0 = rho0[i], r1 = rho1[i];
             bx = (float)(b(r1, rho1[i + ldz]) - b(r0, rho0[i + ldz]));
             bz = (float)(b(r1, rho1[i + 1]) - b(r0, rho0[i + 1]));
-            kc = (float)(t * r1 * v1 * v1 - t * r0 * v0 * v0);
+            // both products rounded (a fused multiply-add would leave one's rounding error where the
+            // models are the same)
+            kc = (float)(__dmul_rn(__dmul_rn(__dmul_rn(t, r1), v1), v1) - __dmul_rn(__dmul_rn(__dmul_rn(t, r0), v0), v0));
         }
         dcbx[i] = bx;
         dcbz[i] = bz;
         dck[i] = kc;
     }
+}
+
+// Where the coefficients of two models differ (FwdArgs::dseg): one warp per column x and 128 rows.
+__global__ void __launch_bounds__(256) k_material_segs(Mat m, Mat m1, const float *__restrict__ dcbx, const float *__restrict__ dcbz,
+                                                       const float *__restrict__ dck, int ntx, int ntz, int ldz, unsigned char *dseg, int *count)
+{
+    const int x = blockIdx.y * 8 + threadIdx.y;
+    if (x >= ntx) return;
+    bool v = false, p = false;
+    for (int k = 0; k < 4; k++) {
+        const int z = blockIdx.x * 128 + 32 * k + threadIdx.x;
+        if (z >= ntz) continue;
+        const size_t i = (size_t)x * ldz + z;
+        v |= !(m1.cbx[i] == m.cbx[i] && m1.cbz[i] == m.cbz[i] && dcbx[i] == 0.f && dcbz[i] == 0.f);
+        p |= !(m1.ck[i] == m.ck[i] && dck[i] == 0.f);
+    }
+    const unsigned bits = (__any_sync(0xffffffffu, v) ? 1u : 0u) | (__any_sync(0xffffffffu, p) ? 2u : 0u);
+    if (threadIdx.x == 0) dseg[(size_t)x * gridDim.x + blockIdx.x] = (unsigned char)bits;
+    if (threadIdx.x == 0 && bits) atomicAdd(count, __popc(bits));
 }
 
 // model_in_pml (acoustic_HLVSPRTMC.cpp:1428-1468): x-edges for interior rows, then z-edges; one
@@ -756,10 +778,18 @@ static void launch_fwd_v(const FwdArgs &a, int nw, dim3 grid, cudaStream_t s, bo
     const bool ck = a.ck.every > 0;
     // register-bound variant of the plain single-wavefield kernel (stencil order 4)
     if constexpr (LC == 4) {
-        if (nw == 1 && !ck && mb == 6) return launch_step(k_fwd_v<4, 1, false, false, false, 6>, grid, s, pdl, a);
+        if (a.ahead && !ck) {
+            if (nw == 2 && a.dseg) return launch_step(k_fwd_v<4, 2, false, false, 2, 0, true>, grid, s, pdl, a);
+            if (nw == 2 && a.dck) return launch_step(k_fwd_v<4, 2, false, false, 1, 0, true>, grid, s, pdl, a);
+            if (nw == 2) return launch_step(k_fwd_v<4, 2, false, false, 0, 0, true>, grid, s, pdl, a);
+            if (mb == 6) return launch_step(k_fwd_v<4, 1, false, false, 0, 6, true>, grid, s, pdl, a);
+        }
+        if (nw == 1 && !ck && mb == 6) return launch_step(k_fwd_v<4, 1, false, false, 0, 6>, grid, s, pdl, a);
     }
-    if (nw == 2 && a.dck) {
-        launch_step(k_fwd_v<LC, 2, false, false, true>, grid, s, pdl, a);
+    if (nw == 2 && a.dseg) {
+        launch_step(k_fwd_v<LC, 2, false, false, 2>, grid, s, pdl, a);
+    } else if (nw == 2 && a.dck) {
+        launch_step(k_fwd_v<LC, 2, false, false, 1>, grid, s, pdl, a);
     } else if (nw == 2) {
         if (ck) launch_step(k_fwd_v<LC, 2, true>, grid, s, pdl, a);
         else launch_step(k_fwd_v<LC, 2, false>, grid, s, pdl, a);
@@ -775,10 +805,18 @@ static void launch_fwd_p(const FwdArgs &a, int nw, dim3 grid, cudaStream_t s, bo
     const bool born = a.s0_out || a.dkappa;
     // register-bound variants of the plain single-wavefield kernel (stencil order 4 only)
     if constexpr (LC == 4) {
+        if (a.ahead && !born && !a.ds.buf && !mb) {
+            if (nw == 2 && a.dseg) return launch_step(k_fwd_p<4, 2, FP_SCAT_SEG, false, 0, true>, grid, s, pdl, a);
+            if (nw == 2 && a.dck) return launch_step(k_fwd_p<4, 2, FP_SCAT, false, 0, true>, grid, s, pdl, a);
+            if (nw == 2) return launch_step(k_fwd_p<4, 2, FP_PLAIN, false, 0, true>, grid, s, pdl, a);
+            return launch_step(k_fwd_p<4, 1, FP_PLAIN, false, 0, true>, grid, s, pdl, a);
+        }
         if (nw == 1 && !a.ds.buf && !born && mb == 4) return launch_step(k_fwd_p<4, 1, FP_PLAIN, false, 4>, grid, s, pdl, a);
         if (nw == 1 && !a.ds.buf && !born && mb == 6) return launch_step(k_fwd_p<4, 1, FP_PLAIN, false, 6>, grid, s, pdl, a);
     }
-    if (nw == 2 && a.dck) {
+    if (nw == 2 && a.dseg) {
+        launch_step(k_fwd_p<LC, 2, FP_SCAT_SEG>, grid, s, pdl, a);
+    } else if (nw == 2 && a.dck) {
         launch_step(k_fwd_p<LC, 2, FP_SCAT>, grid, s, pdl, a);
     } else if (nw == 2) {
         if (born) launch_step(k_fwd_p<LC, 2, FP_BORN>, grid, s, pdl, a);
@@ -800,6 +838,7 @@ template <int LC>
 static void launch_bwd_v(const BwdArgs &a, dim3 grid, cudaStream_t s, bool pdl = false, int mb = 0)
 {
     if constexpr (LC == 4) {   // register-bound variant (stencil order 4)
+        if (mb == 6 && a.ahead) return launch_step(k_bwd_v<4, false, 6, true>, grid, s, pdl, a);
         if (mb == 6) return launch_step(k_bwd_v<4, false, 6>, grid, s, pdl, a);
     }
     launch_step(k_bwd_v<LC>, grid, s, pdl, a);
@@ -943,6 +982,7 @@ static void launch_bwd_p(const BwdArgs &a, dim3 grid, cudaStream_t s, bool pdl =
     if constexpr (LC == 4) {
         if (mb == 4) return launch_step(k_bwd_p<4, false, 4>, grid, s, pdl, a);
         if (mb == 6) return launch_step(k_bwd_p<4, false, 6>, grid, s, pdl, a);
+        if (a.ahead) return launch_step(k_bwd_p<4, false, 0, true>, grid, s, pdl, a);
     }
     launch_step(k_bwd_p<LC>, grid, s, pdl, a);
 }
@@ -1440,6 +1480,7 @@ static int run_forward(swd_ctx *ctx, FwdJob &J, ShotPlan &P)
         a.dcbx = F(ctx->dmat[0]);
         a.dcbz = F(ctx->dmat[1]);
         a.dck = F(ctx->dmat[2]);
+        a.dseg = ctx->scatter_dense ? nullptr : (const unsigned char *)ctx->dseg.p;
     }
     const dim3 grid = grid_blocks(ctx);
     if (J.save_strips) {
@@ -1462,6 +1503,9 @@ static int run_forward(swd_ctx *ctx, FwdJob &J, ShotPlan &P)
     a.wav0 = F(ctx->wav);
     a.wav1 = J.twin ? F(ctx->wav) + nt : F(ctx->wav);
     const int nw = J.twin ? 2 : 1;
+    // (the marches and the on-chip loops take none of these; one field's step kernels gain from
+    // 5.5 M cells on, 4001 x 1601 69.0 -> 62.1 us, two fields' from 2.8 M)
+    a.ahead = streams_hbm(ctx, nw == 2 ? 12 : 6) ? 1 : 0;
     ResPlan rp;
     // Born modelling on the chip, in pieces of the checkpoint interval (RES_PIECE)
     if (a.dkappa && nw == 2 && !a.s0_out && !a.ds.buf && !a.strips.buf && (!a.ck.every || a.ck.every >= RES_PIECE) &&
@@ -2181,14 +2225,24 @@ int swd_set_scatter_model(swd_ctx *ctx, const float *vp1, const float *rho1)
     CKR(grid_to_dev(ctx, F(ctx->rho1), rho1));
     for (auto &b : ctx->mat1) CKR(ensure_grid(ctx, b, sizeof(float)));
     for (auto &b : ctx->dmat) CKR(ensure_grid(ctx, b, sizeof(float)));
+    const dim3 grid = grid_blocks(ctx);
+    CKR(ensure(ctx, ctx->dseg, (size_t)ctx->ntx * grid.x));
+    CKR(ensure(ctx, ctx->ctrl, 64));
+    CK(cudaMemsetAsync(ctx->ctrl.p, 0, 64, ctx->stream));
     k_material<<<592, 256, 0, ctx->stream>>>(F(ctx->vp1), F(ctx->rho1), ctx->grid.dt, ctx->ntx, ctx->ntz, ctx->ldz,
                                              F(ctx->mat1[0]), F(ctx->mat1[1]), F(ctx->mat1[2]), F(ctx->mat1[3]));
     k_material_delta<<<592, 256, 0, ctx->stream>>>(F(ctx->vp), F(ctx->rho), F(ctx->vp1), F(ctx->rho1), ctx->grid.dt,
                                                    ctx->ntx, ctx->ntz, ctx->ldz, F(ctx->dmat[0]), F(ctx->dmat[1]),
                                                    F(ctx->dmat[2]));
-    ctx->launches += 2;
+    k_material_segs<<<grid, dim3(32, 8), 0, ctx->stream>>>(make_mat(ctx), make_mat1(ctx), F(ctx->dmat[0]), F(ctx->dmat[1]),
+                                                           F(ctx->dmat[2]), ctx->ntx, ctx->ntz, ctx->ldz,
+                                                           (unsigned char *)ctx->dseg.p, I32(ctx->ctrl));
+    ctx->launches += 3;
     CK(cudaGetLastError());
+    int nset = 0;
+    CK(cudaMemcpyAsync(&nset, ctx->ctrl.p, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
+    ctx->scatter_dense = (size_t)nset > (size_t)ctx->ntx * grid.x;   // of two bits each
     ctx->have_scatter = true;
     return SWD_OK;
 }
@@ -2388,6 +2442,7 @@ static int rtm_backward_part(swd_ctx *ctx, const swd_shot *shot, const float *da
     }
     BwdArgs b;
     memset(&b, 0, sizeof b);
+    b.ahead = streams_hbm(ctx, 12) ? 1 : 0;
     b.g = make_geo(ctx);
     b.c = make_cpml(ctx);
     b.vp = F(ctx->vp);
