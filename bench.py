@@ -1109,8 +1109,8 @@ def run_decon(args, rank, world, dist):
         "roofline": {"bound": "hbm", "kernel": "decon_window + decon_gather", "achieved": nbytes / (ms * 1e6),
                      "peak": hbm, "peak_source": src, "unit": "GB/s", "frac": nbytes / (ms * 1e6) / hbm,
                      "traffic": None, "algorithmic_bytes_per_launch": nbytes,
-                     "note": "the window transforms are one-warp FP32 FFTs in registers and shared memory (Bluestein's "
-                             "chirp-z through a power-of-two FFT for the odd lengths); HBM is not the bound",
+                     "note": "windows of the reference's padding: real cosine and sine products in shared memory, bound by "
+                             "FP32 FMAs; other lengths, and iterations: one-warp FP32 FFTs; HBM is not the bound",
                      "fft_equivalent_gflops": decon_flops(lay) / (ms * 1e6)},
         "gpu_launches": launches,
         "clocks": clk.summary(),

@@ -1,5 +1,7 @@
 // decon.cuh -- windowed wavenumber-domain PSF deconvolution (decon2d_mine's window loop,
-// kkdecon_acoustic/kk_decon_interp_psf_minewindow.cpp:543-674) as one CTA per window.
+// kkdecon_acoustic/kk_decon_interp_psf_minewindow.cpp:543-674) as one CTA per window.  swd_decon
+// takes the matrix products of decon_dense.cuh for the reference's padding; these kernels do other
+// transform lengths, the iterations, windows too large for those, and swd_decon_noalloc.
 //
 // Per window, in shared memory:
 //   Z = M/|M|_1 + i*S/|S|_1 on an n0 x n1 buffer (M: filterwin^2 image patch centred at

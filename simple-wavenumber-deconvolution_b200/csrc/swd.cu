@@ -1372,11 +1372,30 @@ static MWave march_wave(swd_ctx *c, int k, int in_par)
     return w;
 }
 
-// One-wavefield forward pass by marches; a holds the plain kernels' arguments.  The final state
-// ends in wave[0].
+// The march's own buffers, the second copy of the field and the ring of FP32 strips.  False, with the
+// memory given back, when they do not fit: the step kernels need neither.
+static bool march_room(swd_ctx *ctx, const FwdArgs &a)
+{
+    bool ok = zero_wave2(ctx, 0) == SWD_OK;
+    if (ok && a.strips.buf && a.strips.prec)
+        ok = ensure(ctx, ctx->marchr, sizeof(float) * (size_t)MARCH_RING * a.strips.slen) == SWD_OK;
+    if (ok) return true;
+    cudaGetLastError();
+    cudaStreamSynchronize(ctx->stream);
+    auto drop = [](DevBuf &b) {
+        if (b.p) cudaFree(b.p);
+        b.p = nullptr;
+        b.n = 0;
+    };
+    for (auto &b : ctx->wave2[0]) drop(b);
+    drop(ctx->marchr);
+    return false;
+}
+
+// One-wavefield forward pass by marches (after march_room); a holds the plain kernels' arguments.
+// The final state ends in wave[0].
 static int run_forward_march(swd_ctx *ctx, const FwdArgs &a, ShotPlan &P)
 {
-    CKR(zero_wave2(ctx, 0));
     MFwdArgs m;
     memset(&m, 0, sizeof m);
     m.g = a.g; m.c = a.c; m.m = a.m; m.itp = a.itp; m.wav0 = a.wav0; m.sx = a.sx; m.sz = a.sz;
@@ -1409,7 +1428,6 @@ static int run_forward_march(swd_ctx *ctx, const FwdArgs &a, ShotPlan &P)
         nlist = (int)list.size();
         CKR(ensure(ctx, ctx->marchl, sizeof(int) * nlist));
         CK(cudaMemcpyAsync(ctx->marchl.p, list.data(), sizeof(int) * nlist, cudaMemcpyHostToDevice, ctx->stream));
-        CKR(ensure(ctx, ctx->marchr, sizeof(float) * (size_t)MARCH_RING * a.strips.slen));
         m.strip = F(ctx->marchr);
         m.slen = a.strips.slen;
         m.ring = MARCH_RING;
@@ -1553,7 +1571,8 @@ static int run_forward(swd_ctx *ctx, FwdJob &J, ShotPlan &P)
         CKR(run_resident(ctx, r, rp, a.s0_out ? 3 : 0, &ran));
         if (ran) return SWD_OK;
     }
-    if (nw == 1 && !a.ck.every && !a.ds.buf && !a.s0_out && !a.dkappa && !a.dck && march_ok(ctx)) return run_forward_march(ctx, a, P);
+    if (nw == 1 && !a.ck.every && !a.ds.buf && !a.s0_out && !a.dkappa && !a.dck && march_ok(ctx) && march_room(ctx, a))
+        return run_forward_march(ctx, a, P);
     // one wavefield without checkpoints: the velocity kernel with TMA-staged pressure
     // the plain single-wavefield forward (RTM forward, modelling without a twin): variants of the
     // velocity and pressure launches, chosen by the tuner when SWD_OPT_AUTOTUNE is on
