@@ -310,6 +310,7 @@ extern "C" {
 int swd_rtm_batch(swd_ctx *ctx, int nshots, const swd_shot *shots, const float *const *ricks, const float *const *data,
                   unsigned flags)
 {
+    InCall call(ctx);
     CKR(check_ready(ctx));
     if (nshots < 0 || (nshots > 0 && (!shots || !ricks || !data))) return fail(ctx, SWD_ERR_ARG, "bad batch");
     if (flags & (SWD_RTM_ILLUM_RCV | SWD_RTM_NO_STACK))

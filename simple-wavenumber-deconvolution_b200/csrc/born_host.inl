@@ -183,6 +183,7 @@ static int born_call(swd_ctx *ctx, const swd_shot *shot, const float *rick, cons
 int swd_born(swd_ctx *ctx, const swd_shot *shot, const float *rick, const float *dkappa, float *dseis, void *ckpt,
              size_t ckpt_bytes)
 {
+    InCall call(ctx);
     CKR(born_call(ctx, shot, rick, dkappa, dseis, ckpt, ckpt_bytes));
     return resident_failed(ctx) ? born_call(ctx, shot, rick, dkappa, dseis, ckpt, ckpt_bytes) : SWD_OK;
 }
@@ -285,6 +286,7 @@ static int born_adjoint_call(swd_ctx *ctx, const swd_shot *shot, const float *ri
 int swd_born_adjoint(swd_ctx *ctx, const swd_shot *shot, const float *rick, const float *resid, double *grad,
                      const void *ckpt, size_t ckpt_bytes)
 {
+    InCall call(ctx);
     CKR(born_adjoint_call(ctx, shot, rick, resid, grad, ckpt, ckpt_bytes));
     return resident_failed(ctx) ? born_adjoint_call(ctx, shot, rick, resid, grad, ckpt, ckpt_bytes) : SWD_OK;
 }

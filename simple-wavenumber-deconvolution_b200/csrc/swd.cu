@@ -12,6 +12,7 @@
 #include <algorithm>
 #include <initializer_list>
 #include <cmath>
+#include <atomic>
 #include <mutex>
 #include <string>
 #include <utility>
@@ -1230,27 +1231,41 @@ static bool default_steps(const swd_ctx *c)
 }
 
 // ---- on-chip time loops (resident.cuh) ---------------------------------------------------
-// Whether the context's options ask for nothing but the default step kernels and the grid's
-// wavefields fit on the chip; plan receives the tiling for nw wavefields.  The plain kernels keep
-// every other case: larger grids, other stencil lengths, 16-bit strips, profiling, the kernel
-// variants the options select.
-static bool resident_plan(const swd_ctx *c, int nw, ResPlan *plan, bool born = false)
-{
-    if (!c->use_resident || !c->coop || c->Lc != RES_LC || !c->use_graphs || !default_steps(c)) return false;
-    return res_plan(c->ntx, c->ntz, c->nsm, c->smem_max, nw, born, plan);
-}
-
 // Two of these launches must not share the device (each would hold SMs the other waits for), so
 // every launch waits on the device for the previous one of this process: one event per device.
 struct ResGate {
     std::mutex m;
     cudaEvent_t ev = nullptr;
+    std::atomic<int> calls{0};   // propagation calls in progress
 };
 
 static ResGate &res_gate(int dev)
 {
     static ResGate gates[64];
     return gates[dev & 63];
+}
+
+// A propagation call in progress on the context's device.
+struct InCall {
+    std::atomic<int> *n;
+    explicit InCall(const swd_ctx *c) : n(c ? &res_gate(c->dev).calls : nullptr) { if (n) ++*n; }
+    ~InCall() { if (n) --*n; }
+    InCall(const InCall &) = delete;
+    InCall &operator=(const InCall &) = delete;
+};
+
+// Whether the context's options ask for nothing but the default step kernels and the grid's
+// wavefields fit on the chip; plan receives the tiling for nw wavefields.  The plain kernels keep
+// every other case: larger grids, other stencil lengths, 16-bit strips, profiling, the kernel
+// variants the options select, and calls beside another one on the device: engines of a pool overlap
+// their step kernels, but these launches take turns (us per step and shot, on the chip / step kernels:
+// RTM 401 x 201 one engine 9.4 / 17.0, two 9.3 / 9.8, three 9.3 / 7.2; 801 x 401 13.7 / 19.4, 13.6 /
+// 12.6, 13.5 / 9.9; Born and adjoint 801 x 401 23.9 / 29.1, 23.0 / 20.1, 22.7 / 15.9).  Same bits.
+static bool resident_plan(const swd_ctx *c, int nw, ResPlan *plan, bool born = false)
+{
+    if (res_gate(c->dev).calls > 1) return false;
+    if (!c->use_resident || !c->coop || c->Lc != RES_LC || !c->use_graphs || !default_steps(c)) return false;
+    return res_plan(c->ntx, c->ntz, c->nsm, c->smem_max, nw, born, plan);
 }
 
 // One pass of a.nsteps steps from a.t0.  *ran is false when the launch was refused (fewer SMs than
@@ -2222,6 +2237,7 @@ static int forward_call(swd_ctx *ctx, const swd_shot *shot, const float *rick, c
 int swd_forward(swd_ctx *ctx, const swd_shot *shot, const float *rick, const float *hrick, const float *kz_coef,
                 float *seis, float *seis_up, float *seis_down)
 {
+    InCall call(ctx);
     CKR(forward_call(ctx, shot, rick, hrick, kz_coef, seis, seis_up, seis_down));
     return resident_failed(ctx) ? forward_call(ctx, shot, rick, hrick, kz_coef, seis, seis_up, seis_down) : SWD_OK;
 }
@@ -2269,6 +2285,7 @@ int swd_set_scatter_model(swd_ctx *ctx, const float *vp1, const float *rho1)
 int swd_forward_scatter(swd_ctx *ctx, const swd_shot *shot, const float *rick, const float *hrick,
                         const float *kz_coef, float *seis, float *seis_up, float *seis_down)
 {
+    InCall call(ctx);
     CKR(check_ready(ctx));
     if (!ctx->have_scatter) return fail(ctx, SWD_ERR_STATE, "no perturbed model (swd_set_scatter_model)");
     if (!rick || !seis) return fail(ctx, SWD_ERR_ARG, "rick and seis are required");
@@ -2652,6 +2669,7 @@ static int rtm_backward_part(swd_ctx *ctx, const swd_shot *shot, const float *da
 int swd_rtm_shot(swd_ctx *ctx, const swd_shot *shot, const float *rick, const float *data, unsigned flags, float *syn,
                  float *image_pp, float *image_src, float *fimage)
 {
+    InCall call(ctx);
     CKR(check_ready(ctx));
     if (!rick || !data) return fail(ctx, SWD_ERR_ARG, "rick and data are required");
     CKR(rtm_forward_part(ctx, shot, rick, syn));
@@ -2663,6 +2681,7 @@ int swd_rtm_shot(swd_ctx *ctx, const swd_shot *shot, const float *rick, const fl
 
 int swd_rtm_forward(swd_ctx *ctx, const swd_shot *shot, const float *rick, float *syn)
 {
+    InCall call(ctx);
     CKR(check_ready(ctx));
     if (!rick) return fail(ctx, SWD_ERR_ARG, "rick is required");
     CKR(rtm_forward_part(ctx, shot, rick, syn));
@@ -2678,6 +2697,7 @@ int swd_rtm_forward(swd_ctx *ctx, const swd_shot *shot, const float *rick, float
 int swd_rtm_backward(swd_ctx *ctx, const swd_shot *shot, const float *data, unsigned flags, float *image_pp,
                      float *image_src, float *fimage)
 {
+    InCall call(ctx);
     CKR(check_ready(ctx));
     if (!data) return fail(ctx, SWD_ERR_ARG, "data is required");
     const swd_ctx::KeptShotState kept = ctx->kept;

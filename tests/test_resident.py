@@ -5,6 +5,8 @@ tiles, one tile only along z, the smallest grid, one and two columns per warp at
 ranges, the largest grid that fits; receivers scattered over the whole padded grid (several per
 warp and per cell column, duplicates, frame cells), the source inside the strip band and in the
 frame.  The arithmetic is the same term by term, so the comparison is exact."""
+from concurrent.futures import ThreadPoolExecutor
+
 import numpy as np
 import pytest
 import torch
@@ -118,3 +120,28 @@ def test_resident_born_same_bits(swd, name):
     for i, (a, b) in enumerate(zip(out[1], out[0])):
         assert np.abs(b).max() > 0, i
         assert np.array_equal(a, b), i
+
+
+def test_engines_side_by_side_same_bits(swd):
+    """Engines that run at the same time (their calls choose the step kernels while another call is in
+    progress) give what one engine gives alone."""
+    nt = 150
+    made = [_engine(swd, 100, 100, 10, nt, 3) for _ in range(3)]
+    ntx, ntz = made[0][2]
+    rng = np.random.default_rng(8)
+    s = swd.ShotSpec(60, 20, np.full(40, 70, np.int32), np.arange(20, 60).astype(np.int32), nt)
+    rick, data = swd.ricker_wave(nt, 25.0, 5e-4), rng.standard_normal((40, nt)).astype(np.float32)
+
+    def shots(E, n):
+        r = []
+        for _ in range(n):
+            E.rtm_shot(s, rick, data, flags=swd.RTM_NO_STACK, want=())
+            r += [E.forward(s, rick)] + list(E.rtm_raw()[:2])
+        return r
+
+    ref = shots(made[0][0], 1)
+    with ThreadPoolExecutor(3) as pool:
+        out = list(pool.map(lambda m: shots(m[0], 6), made))
+    for r in out:
+        for k, a in enumerate(r):
+            assert np.array_equal(a, ref[k % 3])
