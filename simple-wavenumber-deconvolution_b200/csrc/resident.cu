@@ -623,9 +623,9 @@ __global__ void __launch_bounds__(32 * MW, 1) k_resident(const ResArgs a)
             }
 }
 
-bool res_plan(int ntx, int ntz, int nsm, size_t smem_max, int nw, bool born, ResPlan *p)
+bool res_plan(int ntx, int ntz, int pmlc, int nsm, size_t smem_max, int nw, bool born, ResPlan *p)
 {
-    if (ntx < 48 || ntz < 48) return false;   // the strip bands of both sides never meet in a thread's rows
+    if (ntx < 48 || ntz < 48 || !strip_bands_apart(ntz, pmlc, RES_LC)) return false;
     p->nw = nw;
     p->GZ = (ntz + RES_TZ - 1) / RES_TZ;
     const int gx = nsm / p->GZ;

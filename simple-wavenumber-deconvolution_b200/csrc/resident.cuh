@@ -37,6 +37,7 @@
 // results are the same bits.
 #pragma once
 #include "prop.cuh"
+#include "rules.h"
 
 namespace swd {
 
@@ -101,8 +102,8 @@ __host__ __device__ inline size_t res_smem(int TX, int nw)
 // launches nsteps steps; mode 0 forward, 1 backward (plan.nw == 2), 2 Born (plan.nw == 2), 3 forward
 // with S0 (plan.nw == 1); modes 2 and 3 may run a pass in pieces
 cudaError_t res_launch(const ResArgs &a, const ResPlan &p, int mode, cudaStream_t st);
-// tiling of an ntx x ntz grid on nsm SMs with smem_max bytes of shared memory per CTA; false
-// when the wavefields do not fit; born: with the perturbation of mode 2
-bool res_plan(int ntx, int ntz, int nsm, size_t smem_max, int nw, bool born, ResPlan *p);
+// tiling of an ntx x ntz grid (pmlc frame cells) on nsm SMs with smem_max bytes of shared memory per
+// CTA; false when the wavefields do not fit; born: with the perturbation of mode 2
+bool res_plan(int ntx, int ntz, int pmlc, int nsm, size_t smem_max, int nw, bool born, ResPlan *p);
 
 }  // namespace swd

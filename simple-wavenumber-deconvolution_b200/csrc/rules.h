@@ -1,0 +1,13 @@
+// rules.h -- sizes for which the engine takes one kernel path or another: plain host functions of
+// numbers, without CUDA, so that they can be checked over whole ranges of sizes on the CPU.
+#pragma once
+
+namespace swd {
+
+// The on-chip loops and the marches keep one strip offset per thread for its four rows (the rows
+// 4k .. 4k + 3 of the padded grid), so no four rows may hold cells of the top strip and of the bottom
+// strip.  The strips are Lc rows each at both ends of the ntz - 2 pmlc interior rows; from 2 Lc + 3
+// interior rows on, three rows or more lie between them.
+inline bool strip_bands_apart(int ntz, int pmlc, int Lc) { return ntz - 2 * pmlc >= 2 * Lc + 3; }
+
+}  // namespace swd

@@ -1265,7 +1265,7 @@ static bool resident_plan(const swd_ctx *c, int nw, ResPlan *plan, bool born = f
 {
     if (res_gate(c->dev).calls > 1) return false;
     if (!c->use_resident || !c->coop || c->Lc != RES_LC || !c->use_graphs || !default_steps(c)) return false;
-    return res_plan(c->ntx, c->ntz, c->nsm, c->smem_max, nw, born, plan);
+    return res_plan(c->ntx, c->ntz, c->pmlc, c->nsm, c->smem_max, nw, born, plan);
 }
 
 // One pass of a.nsteps steps from a.t0.  *ran is false when the launch was refused (fewer SMs than
@@ -1333,6 +1333,7 @@ static bool resident_failed(swd_ctx *ctx)
 static bool march_ok(const swd_ctx *c)
 {
     return c->use_march && c->Lc == MARCH_LC && default_steps(c) && c->use_graphs && c->stream &&
+           strip_bands_apart(c->ntz, c->pmlc, c->Lc) &&
            (double)c->ntx * c->ldz * sizeof(float) * 6 > 0.8 * (double)c->l2_bytes;
 }
 

@@ -145,3 +145,22 @@ def test_engines_side_by_side_same_bits(swd):
     for r in out:
         for k, a in enumerate(r):
             assert np.array_equal(a, ref[k % 3])
+
+
+@pytest.mark.parametrize("nz,pml", [(9, 30), (9, 17), (10, 17), (11, 17)])
+def test_models_of_few_rows_same_bits(swd, nz, pml):
+    """Models whose top and bottom strips lie within four rows of each other."""
+    nt = 120
+    E, rng, (ntx, ntz) = _engine(swd, 60, nz, pml, nt, 4)
+    pmlc = pml + 4
+    rix, riz = np.full(nz, pmlc + 40, np.int32), (pmlc + np.arange(nz)).astype(np.int32)
+    s = swd.ShotSpec(pmlc + 20, pmlc + 4, rix, riz, nt)
+    rick, data = swd.ricker_wave(nt, 25.0, 5e-4), rng.standard_normal((nz, nt)).astype(np.float32)
+    out = []
+    for res in (0, 1):
+        E.set_option(swd.OPT_RESIDENT, res)
+        r = E.rtm_shot(s, rick, data, flags=swd.RTM_NO_STACK)
+        out.append([r[k] for k in sorted(r)] + list(E.rtm_raw()[:2]))
+    for a, b in zip(*out):
+        assert np.abs(b).max() > 0
+        assert np.array_equal(a, b)

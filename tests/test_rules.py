@@ -1,0 +1,48 @@
+"""The size rules that choose a kernel path (csrc/rules.h), over whole ranges of sizes on the CPU."""
+import ctypes as C
+import subprocess
+
+import pytest
+
+from conftest import PKG_DIR
+
+WRAP = """
+#include "rules.h"
+extern "C" {
+int bands_apart(int ntz, int pmlc, int Lc) { return swd::strip_bands_apart(ntz, pmlc, Lc); }
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def rules(tmp_path_factory):
+    d = tmp_path_factory.mktemp("rules")
+    (d / "wrap.cpp").write_text(WRAP)
+    subprocess.run(["g++", "-std=c++17", "-O1", "-Wall", "-Werror", "-shared", "-fPIC", f"-I{PKG_DIR / 'csrc'}",
+                    "-o", str(d / "rules.so"), str(d / "wrap.cpp")], check=True)
+    return C.CDLL(str(d / "rules.so"))
+
+
+def test_strip_rows_of_a_thread(rules):
+    """Wherever the rule lets a grid through, the strip slot a thread forms from its single offset is
+    the cell's own slot, and no grid of 11 or more interior rows is turned away."""
+    Lc, nx, ix = 4, 20, 7
+    wrong = set()
+    for nz in range(9, 16):
+        for pml in range(1, 45):
+            p = pml + Lc
+            ntz = nz + 2 * p
+            ok = True
+            for z0 in range(0, ntz, 4):
+                off, own = 0, {}
+                for z in range(z0, min(z0 + 4, ntz)):
+                    if p <= z < p + Lc:                          # top strip: Lc values per column
+                        off, own[z] = z0 - p, z - p
+                    elif ntz - p - Lc <= z < ntz - p:            # bottom strip, after the top one
+                        off, own[z] = Lc * nx + z0 - (ntz - p - Lc), Lc * nx + z - (ntz - p - Lc)
+                ok &= all(off + ix * Lc + z - z0 == s + ix * Lc for z, s in own.items())
+            if not ok:
+                wrong.add(nz)
+            assert rules.bands_apart(ntz, p, Lc) == (nz >= 11)
+            assert ok or nz < 11, (nz, pml)
+    assert wrong == {9, 10}   # the check does see the grids that must be turned away
