@@ -10,4 +10,9 @@ namespace swd {
 // interior rows on, three rows or more lie between them.
 inline bool strip_bands_apart(int ntz, int pmlc, int Lc) { return ntz - 2 * pmlc >= 2 * Lc + 3; }
 
+// A march forms its cell index, column times row pitch plus row, in 32 bits (a lane's address is then
+// one multiply-add per array).  Grids beyond that keep the step kernels: two copies of the field and
+// six more arrays of 2^31 cells leave no room on a device of 180 GB for anything else.
+inline bool march_index_fits(int ntx, int ldz) { return (long long)ntx * ldz <= 0x7fffffffLL; }
+
 }  // namespace swd

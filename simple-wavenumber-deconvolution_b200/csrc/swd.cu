@@ -1333,7 +1333,7 @@ static bool resident_failed(swd_ctx *ctx)
 static bool march_ok(const swd_ctx *c)
 {
     return c->use_march && c->Lc == MARCH_LC && default_steps(c) && c->use_graphs && c->stream &&
-           strip_bands_apart(c->ntz, c->pmlc, c->Lc) &&
+           strip_bands_apart(c->ntz, c->pmlc, c->Lc) && march_index_fits(c->ntx, c->ldz) &&
            (double)c->ntx * c->ldz * sizeof(float) * 6 > 0.8 * (double)c->l2_bytes;
 }
 

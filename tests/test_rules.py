@@ -10,6 +10,7 @@ WRAP = """
 #include "rules.h"
 extern "C" {
 int bands_apart(int ntz, int pmlc, int Lc) { return swd::strip_bands_apart(ntz, pmlc, Lc); }
+int index_fits(int ntx, int ldz) { return swd::march_index_fits(ntx, ldz); }
 }
 """
 
@@ -46,3 +47,12 @@ def test_strip_rows_of_a_thread(rules):
             assert rules.bands_apart(ntz, p, Lc) == (nz >= 11)
             assert ok or nz < 11, (nz, pml)
     assert wrong == {9, 10}   # the check does see the grids that must be turned away
+
+
+def test_march_index_range(rules):
+    """Every index a march forms (col * ldz + row, row from -8 to ldz - 4) fits in 32 bits where the
+    rule lets the grid through; the largest grid that fits is let through."""
+    for ldz in (64, 1696, 46336, 46368, 65536, 1 << 20):
+        for ntx in (100, 4069, (2 ** 31 - 1) // ldz, (2 ** 31 - 1) // ldz + 1, 46341, 2 ** 31 // ldz + 100):
+            fits = (ntx - 1) * ldz + ldz - 4 < 2 ** 31 and ntx * ldz < 2 ** 31
+            assert bool(rules.index_fits(ntx, ldz)) == fits, (ntx, ldz)
