@@ -406,6 +406,10 @@ int swd_set_option(swd_ctx *ctx, int option, int value)
             if (value != 0 && value != 1) return fail(ctx, SWD_ERR_ARG, "SWD_OPT_RESIDENT takes 0 or 1");
             ctx->use_resident = value;
             return SWD_OK;
+        case SWD_OPT_RESIDENT_STOP:
+            if (value < -1) return fail(ctx, SWD_ERR_ARG, "SWD_OPT_RESIDENT_STOP takes -1, 0 or a number of steps");
+            ctx->res_stop = value;
+            return SWD_OK;
         case SWD_OPT_LEAN:
             if (value != 0 && value != 1) return fail(ctx, SWD_ERR_ARG, "SWD_OPT_LEAN takes 0 or 1");
             ctx->use_lean = value;
@@ -431,6 +435,7 @@ int swd_get_option(swd_ctx *ctx, int option, int *value)
         case SWD_OPT_LEAN: *value = ctx->use_lean; return SWD_OK;
         case SWD_OPT_MARCH: *value = ctx->use_march; return SWD_OK;
         case SWD_OPT_RESIDENT: *value = ctx->use_resident; return SWD_OK;
+        case SWD_OPT_RESIDENT_STOP: *value = ctx->res_stop; return SWD_OK;
         case SWD_OPT_TUNED_FWD: *value = ctx->autotune && ctx->tfwd.choice >= 0 ? ctx->tfwd.cand[ctx->tfwd.choice] : -1; return SWD_OK;
         case SWD_OPT_TUNED_BWD: *value = ctx->autotune && ctx->tbwd.choice >= 0 ? ctx->tbwd.cand[ctx->tbwd.choice] : -1; return SWD_OK;
         default: return fail(ctx, SWD_ERR_ARG, "unknown option %d", option);

@@ -72,7 +72,8 @@ __global__ void __launch_bounds__(32 * MW, 1) k_resident(const ResArgs a)
     const bool hl = bx > 0, hr = bx < GX - 1, ht = bz > 0, hb = bz < GZ - 1;
     const int ntx = g.ntx, ntz = g.ntz, ldz = g.ldz;
 
-    if (*a.err) return;   // an earlier pass gave up: do not wait for anyone
+    // an earlier pass gave up: do not wait for anyone
+    if (*a.err || (a.stop < 0 && blockIdx.x == 0)) return;
     extern __shared__ float4 smem4[];
     float *sm = (float *)smem4;
     const int psz = (TX + 8) * PZ, vsz = (TX + 8) * TZ;
@@ -600,13 +601,15 @@ __global__ void __launch_bounds__(32 * MW, 1) k_resident(const ResArgs a)
         if (s + 1 < a.nsteps) receive(tab + tabcap, nP, tag);
         if (__syncthreads_or(bad)) break;
     }
-    if (__syncthreads_or(bad)) {
+    if (__syncthreads_or(bad || (a.stop > 0 && blockIdx.x == 0))) {
         if (tid == 0) { *a.err = 1; *(volatile int *)a.host_err = 1; }
         return;
     }
-    // ---- final state
+    // ---- final state.  None after a backward pass: nobody reads it, and where a tile gave up in one of
+    // the last steps the pass runs again from the forward pass's final fields, which the tiles that got
+    // through must not have overwritten.
 #pragma unroll
-    for (int k = 0; k < NW; k++)
+    for (int k = 0; k < (MODE == 1 ? 0 : NW); k++)
 #pragma unroll
         for (int i = 0; i < XR; i++)
             if (has(i)) {

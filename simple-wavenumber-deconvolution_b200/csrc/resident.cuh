@@ -46,7 +46,7 @@ constexpr int RES_TZ = 128;          // rows of a tile (32 lanes x 4)
 constexpr int RES_PZ = RES_TZ + 8;   // pressure column in shared memory with its halo rows
 constexpr int RES_MAXW1 = 16;        // warps of a CTA at most, one column per warp
 constexpr int RES_MAXW2 = 12;        // two columns per warp; one column with the larger register budget
-constexpr int RES_SPIN = 1 << 22;
+constexpr int RES_SPIN = 1 << 22;    // tries of a wait, 0.36 us each
 // Steps of a piece at least: Born passes stop at every checkpoint, and a launch that loads and
 // stores the whole state costs about 15 to 25 us.  Born plus adjoint pass per step with checkpoints
 // every 4 / 8 / 64 steps: 401 x 201 31.2 -> 27.1 / 27.8 -> 21.8 / 24.9 -> 17.4 us, 801 x 401
@@ -82,6 +82,9 @@ struct ResArgs {
     int TX, GX, GZ;
     uint4 *ll;             // exchange words
     unsigned epoch;        // tag of the step before the first
+    // tests of the recovery: 1 the first tile reports at the end that it gave up, -1 it does not start
+    // and its neighbours wait for it in vain; 0: neither
+    int stop;
     int *err, *host_err;   // set when a wait gave up; *err also keeps later launches from starting
 };
 

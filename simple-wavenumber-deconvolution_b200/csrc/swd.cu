@@ -131,6 +131,7 @@ struct swd_ctx {
     unsigned res_epoch = 0;
     volatile int *res_flag = nullptr;
     int use_resident = 1;         // SWD_OPT_RESIDENT
+    int res_stop = 0;             // SWD_OPT_RESIDENT_STOP
     int use_march = 1;            // SWD_OPT_MARCH
     DevBuf marchl, marcht, marchr;   // strip blocks, tasks, ring of FP32 strips of a marching pass
     int nsm = 0, coop = 0;
@@ -1299,6 +1300,8 @@ static int run_resident(swd_ctx *ctx, ResArgs &a, const ResPlan &p, int mode, bo
     a.GX = p.GX;
     a.GZ = p.GZ;
     a.epoch = ctx->res_epoch;
+    a.stop = ctx->res_stop > 0 ? 1 : ctx->res_stop;
+    if (ctx->res_stop > 0) a.nsteps = std::min(a.nsteps, ctx->res_stop);
     ctx->res_epoch += (unsigned)a.nsteps + 1u;
     ResGate &gate = res_gate(ctx->dev);
     std::lock_guard<std::mutex> hold(gate.m);

@@ -164,3 +164,86 @@ def test_models_of_few_rows_same_bits(swd, nz, pml):
     for a, b in zip(*out):
         assert np.abs(b).max() > 0
         assert np.array_equal(a, b)
+
+
+GIVE_UP = ["forward", "twin", "rtm_shot", "rtm_forward", "rtm_backward", "batch", "born", "born_checkpoints", "adjoint", "adjoint_checkpoints"]
+
+
+def _gives_up(swd, grid, name, stops, nt=60):
+    """The call `name` by the step kernels, then on the chip with each SWD_OPT_RESIDENT_STOP in turn, then
+    undisturbed: the same bits (results and stack) every time, and the option reads 0 after a pass that
+    gave up."""
+    nx, nz, pml = GRIDS[grid]
+    E, rng, (ntx, ntz) = _engine(swd, nx, nz, pml, nt, 6)
+    pmlc = pml + 4
+    rix, riz = np.full(20, pmlc + nx // 2, np.int32), (pmlc + np.arange(20)).astype(np.int32)
+    s = swd.ShotSpec(pmlc + nx // 2 - 6, pmlc + 1, rix, riz, nt)
+    rick = swd.ricker_wave(nt, 60.0, 5e-4)
+    hr, coef = E.hilbert(rick), rng.uniform(0.2, 1.0, swd.pow2(ntz)).astype(np.float32)
+    data = rng.standard_normal((20, nt)).astype(np.float32)
+    dk = (rng.standard_normal((ntx, ntz)) * 1e7).astype(np.float32)
+    E.set_checkpointing(16 if name.endswith("checkpoints") else 0, swd.STRIP_F32)
+    ck = torch.empty(max(16, E.checkpoint_bytes(nt)), dtype=torch.uint8, device="cuda") if name.endswith("checkpoints") else None
+
+    def call(stop):
+        E.stack_reset()
+        E.set_option(swd.OPT_RESIDENT_STOP, 0 if name == "rtm_backward" else stop)
+        if name == "forward":
+            return [E.forward(s, rick)]
+        if name == "twin":
+            return list(E.forward(s, rick, hrick=hr, kz_coef=coef))
+        if name == "rtm_shot":
+            o = E.rtm_shot(s, rick, data, want=("image_pp", "image_src", "fimage", "syn"))
+            return [o[k] for k in sorted(o)] + list(E.rtm_raw()[:2]) + [E.stack(edge_zero=False)]
+        if name == "rtm_forward":
+            r = [E.rtm_forward(s, rick, syn=True)]
+            E.set_option(swd.OPT_RESIDENT_STOP, 0)
+            E.rtm_backward(s, data, want=())
+            return r + list(E.rtm_raw()[:2]) + [E.stack(edge_zero=False)]
+        if name == "rtm_backward":
+            E.rtm_forward(s, rick)
+            E.set_option(swd.OPT_RESIDENT_STOP, stop)
+            o = E.rtm_backward(s, data)
+            return [o[k] for k in sorted(o)] + list(E.rtm_raw()[:2]) + [E.stack(edge_zero=False)]
+        if name == "batch":
+            E.rtm_batch([s, s], [rick, rick], [data, 2 * data])
+            return [E.stack(edge_zero=False)]
+        if name.startswith("born"):
+            return [E.born(s, rick, dk, ckpt=ck)] + ([E.born_adjoint(s, rick, data, ckpt=ck)] if ck is not None else [])
+        if ck is not None:
+            E.set_option(swd.OPT_RESIDENT_STOP, 0)
+            E.born(s, rick, dk, ckpt=ck)
+            E.set_option(swd.OPT_RESIDENT_STOP, stop)
+        return [E.born_adjoint(s, rick, data, ckpt=ck)]
+
+    E.set_option(swd.OPT_RESIDENT, 0)
+    ref = call(0)
+    for stop in list(stops) + [0]:
+        E.set_option(swd.OPT_RESIDENT, 1)
+        got = call(stop)
+        assert E.get_option(swd.OPT_RESIDENT) == (1 if stop == 0 else 0)
+        for i, (a, b) in enumerate(zip(got, ref)):
+            assert np.abs(b).max() > 0, (stop, i)
+            assert np.array_equal(a, b), (stop, i)
+
+
+@pytest.mark.parametrize("name", GIVE_UP)
+@pytest.mark.parametrize("grid", ["z_one_row_left", "x_24_columns"])
+def test_pass_that_gives_up_runs_again(swd, grid, name):
+    """Passes that stop after their first step and after some: the call runs again
+    with the step kernels, and a later pass on the chip is not disturbed by the stopped one."""
+    _gives_up(swd, grid, name, (1, 13))
+
+
+@pytest.mark.parametrize("name", ["rtm_shot", "adjoint_checkpoints"])
+def test_waits_that_run_out(swd, name):
+    """One tile does not start: its neighbours wait for its words until their tries run out, and theirs
+    in turn."""
+    _gives_up(swd, "smallest", name, (-1,))
+
+
+def test_stop_option(swd):
+    E = _engine(swd, 20, 20, 10, 16, 1)[0]
+    assert E.get_option(swd.OPT_RESIDENT_STOP) == 0
+    with pytest.raises(swd.SwdError):
+        E.set_option(swd.OPT_RESIDENT_STOP, -2)
