@@ -13,7 +13,6 @@
 #include <initializer_list>
 #include <cmath>
 #include <atomic>
-#include <mutex>
 #include <string>
 #include <utility>
 #include <vector>
@@ -130,6 +129,7 @@ struct swd_ctx {
     DevBuf resll, reserr;
     unsigned res_epoch = 0;
     volatile int *res_flag = nullptr;
+    bool res_running = false;     // a launch of the call in progress may not have ended
     int use_resident = 1;         // SWD_OPT_RESIDENT
     int res_stop = 0;             // SWD_OPT_RESIDENT_STOP
     int use_march = 1;            // SWD_OPT_MARCH
@@ -1232,25 +1232,30 @@ static bool default_steps(const swd_ctx *c)
 }
 
 // ---- on-chip time loops (resident.cuh) ---------------------------------------------------
-// Two of these launches must not share the device (each would hold SMs the other waits for), so
-// every launch waits on the device for the previous one of this process: one event per device.
-struct ResGate {
-    std::mutex m;
-    cudaEvent_t ev = nullptr;
-    std::atomic<int> calls{0};   // propagation calls in progress
-};
-
-static ResGate &res_gate(int dev)
+// Propagation calls in progress on a device.  Two on-chip launches must not share the device (each
+// would hold SMs the other waits for): a call launches them only while it is alone (resident_plan),
+// and is counted until its last one has ended.  A second call that begins meanwhile sees both and
+// takes the step kernels, which run beside an on-chip launch.
+static std::atomic<int> &calls_on(int dev)
 {
-    static ResGate gates[64];
-    return gates[dev & 63];
+    static std::atomic<int> calls[64];
+    return calls[dev & 63];
 }
 
-// A propagation call in progress on the context's device.
+// A propagation call in progress on the context's device.  At its end, on every way out, no on-chip
+// launch is left running.
 struct InCall {
-    std::atomic<int> *n;
-    explicit InCall(const swd_ctx *c) : n(c ? &res_gate(c->dev).calls : nullptr) { if (n) ++*n; }
-    ~InCall() { if (n) --*n; }
+    swd_ctx *c;
+    explicit InCall(swd_ctx *ctx) : c(ctx) { if (c) ++calls_on(c->dev); }
+    ~InCall()
+    {
+        if (!c) return;
+        if (c->res_running) {
+            cudaStreamSynchronize(c->stream);
+            c->res_running = false;
+        }
+        --calls_on(c->dev);
+    }
     InCall(const InCall &) = delete;
     InCall &operator=(const InCall &) = delete;
 };
@@ -1264,7 +1269,7 @@ struct InCall {
 // 12.6, 13.5 / 9.9; Born and adjoint 801 x 401 23.9 / 29.1, 23.0 / 20.1, 22.7 / 15.9).  Same bits.
 static bool resident_plan(const swd_ctx *c, int nw, ResPlan *plan, bool born = false)
 {
-    if (res_gate(c->dev).calls > 1) return false;
+    if (calls_on(c->dev) > 1) return false;
     if (!c->use_resident || !c->coop || c->Lc != RES_LC || !c->use_graphs || !default_steps(c)) return false;
     return res_plan(c->ntx, c->ntz, c->pmlc, c->nsm, c->smem_max, nw, born, plan);
 }
@@ -1303,16 +1308,12 @@ static int run_resident(swd_ctx *ctx, ResArgs &a, const ResPlan &p, int mode, bo
     a.stop = ctx->res_stop > 0 ? 1 : ctx->res_stop;
     if (ctx->res_stop > 0) a.nsteps = std::min(a.nsteps, ctx->res_stop);
     ctx->res_epoch += (unsigned)a.nsteps + 1u;
-    ResGate &gate = res_gate(ctx->dev);
-    std::lock_guard<std::mutex> hold(gate.m);
-    if (!gate.ev) CK(cudaEventCreateWithFlags(&gate.ev, cudaEventDisableTiming));
-    else CK(cudaStreamWaitEvent(ctx->stream, gate.ev, 0));
     if (res_launch(a, p, mode, ctx->stream) != cudaSuccess) {
         cudaGetLastError();
         ctx->use_resident = 0;
         return SWD_OK;
     }
-    CK(cudaEventRecord(gate.ev, ctx->stream));
+    ctx->res_running = true;
     ctx->launches++;
     *ran = true;
     return SWD_OK;

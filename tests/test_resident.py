@@ -5,11 +5,15 @@ tiles, one tile only along z, the smallest grid, one and two columns per warp at
 ranges, the largest grid that fits; receivers scattered over the whole padded grid (several per
 warp and per cell column, duplicates, frame cells), the source inside the strip band and in the
 frame.  The arithmetic is the same term by term, so the comparison is exact."""
+import subprocess
+import sys
 from concurrent.futures import ThreadPoolExecutor
 
 import numpy as np
 import pytest
 import torch
+
+from conftest import ROOT
 
 pytestmark = pytest.mark.gpu
 
@@ -247,3 +251,34 @@ def test_stop_option(swd):
     assert E.get_option(swd.OPT_RESIDENT_STOP) == 0
     with pytest.raises(swd.SwdError):
         E.set_option(swd.OPT_RESIDENT_STOP, -2)
+
+
+RESET = """
+import ctypes, sys
+import numpy as np
+sys.path.insert(0, sys.argv[1])
+from conftest import load_pkg
+swd = load_pkg()
+nt = 40
+def shot(res):
+    E = swd.Engine(100, 60, 10, 4, 5.0, 5.0, 5e-4, nt)
+    vp = np.full((128, 88), 2000.0, np.float32)
+    E.setup_default(vp, np.full_like(vp, 1000.0))
+    E.set_option(swd.OPT_RESIDENT, res)
+    s = swd.ShotSpec(40, 20, np.full(9, 50, np.int32), np.arange(15, 24).astype(np.int32), nt)
+    out = [E.forward(s, swd.ricker_wave(nt, 60.0, 5e-4)) for _ in range(2)]
+    assert E.get_option(swd.OPT_RESIDENT) == res
+    E.close()
+    return out[1]
+ref = shot(0)
+assert np.abs(ref).max() > 0 and np.array_equal(shot(1), ref)
+assert ctypes.CDLL("libcudart.so.12").cudaDeviceReset() == 0
+assert np.array_equal(shot(1), ref)
+"""
+
+
+def test_on_chip_passes_after_a_device_reset(swd):
+    """A program that closes its engines, resets its device context and goes on (in a process of its
+    own): the on-chip passes keep nothing from before."""
+    r = subprocess.run([sys.executable, "-c", RESET, str(ROOT / "tests")], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
