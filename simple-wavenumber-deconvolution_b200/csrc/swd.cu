@@ -1242,8 +1242,10 @@ static std::atomic<int> &calls_on(int dev)
     return calls[dev & 63];
 }
 
+static bool resident_failed(swd_ctx *ctx);
+
 // A propagation call in progress on the context's device.  At its end, on every way out, no on-chip
-// launch is left running.
+// launch is left running and no error word set.
 struct InCall {
     swd_ctx *c;
     explicit InCall(swd_ctx *ctx) : c(ctx) { if (c) ++calls_on(c->dev); }
@@ -1252,6 +1254,7 @@ struct InCall {
         if (!c) return;
         if (c->res_running) {
             cudaStreamSynchronize(c->stream);
+            resident_failed(c);
             c->res_running = false;
         }
         --calls_on(c->dev);

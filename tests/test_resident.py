@@ -253,6 +253,27 @@ def test_stop_option(swd):
         E.set_option(swd.OPT_RESIDENT_STOP, -2)
 
 
+def test_error_after_a_pass_that_gave_up(swd):
+    """A call that returns an error after its on-chip pass gave up leaves nothing behind: the next
+    survey, by the step kernels, is stacked."""
+    nt = 60
+    E, rng, _ = _engine(swd, 100, 100, 10, nt, 6)
+    s = swd.ShotSpec(40, 20, np.full(20, 70, np.int32), np.arange(20, 40).astype(np.int32), nt)
+    rick, data = swd.ricker_wave(nt, 60.0, 5e-4), rng.standard_normal((20, nt)).astype(np.float32)
+    E.set_option(swd.OPT_RESIDENT, 0)
+    E.rtm_shot(s, rick, data)
+    ref = E.stack(edge_zero=False)
+    E.stack_reset()
+    E.set_option(swd.OPT_RESIDENT, 1)
+    E.set_option(swd.OPT_RESIDENT_STOP, 5)
+    with pytest.raises(swd.SwdError):   # angle gathers that were not set up: refused after the forward pass
+        E.rtm_shot(s, rick, data, flags=swd.RTM_PREPROCESS | swd.RTM_CIG)
+    E.set_option(swd.OPT_RESIDENT_STOP, 0)
+    E.set_option(swd.OPT_RESIDENT, 0)
+    E.rtm_batch([s], [rick], [data])
+    assert np.abs(ref).max() > 0 and np.array_equal(E.stack(edge_zero=False), ref)
+
+
 RESET = """
 import ctypes, sys
 import numpy as np
