@@ -78,6 +78,10 @@ __host__ __device__ inline size_t dense_smem(const DenseGeo &d, int h1, int h2)
 }
 __host__ __device__ inline size_t dense_spec(const DenseGeo &d) { return (size_t)d.K1 * (d.NB * d.blk); }   // float4 per PSF
 
+// Shared memory a window's CTA may take, and the limit both kernels are given on every call: it belongs
+// to the kernel on the device, not to a context, so no call may lower it under another thread's launch.
+constexpr int DENSE_SMEM_MAX = 226 * 1024;
+
 // Tables of one axis: C then S, [TR][KT] each, zero for k >= K; double, rounded once.
 __global__ void k_dense_tables(float *t, int L, int K, int TR, int KT)
 {

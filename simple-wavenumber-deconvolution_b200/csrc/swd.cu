@@ -634,6 +634,8 @@ __global__ void k_stack_out(const double *__restrict__ st, float *out, int nx, i
 // indices, rows iz < pml+8 unchanged.  Coefficients come from the host.  The block's cells and
 // their window are converted to double once, in shared memory (8 + 2w columns of 32 + 2w rows):
 // converting at every tap kept the conversion unit busy (1669 x 869, 11 x 11 window: 120 -> 83 us).
+constexpr int SMOOTH_MAX_WINDOW = 64;
+static size_t smooth_smem(int w) { return sizeof(double) * (8 + 2 * (size_t)w) * (32 + 2 * (size_t)w); }
 __global__ void __launch_bounds__(256) k_smooth(const float *__restrict__ vin, float *vout, const double *__restrict__ coef, int ntx,
                                                 int ntz, int pml, int w)
 {
@@ -1862,7 +1864,7 @@ static bool dense_plan(const DeconGeo &g, DenseGeo &d)
     d.TR2 = up8(std::max(d.hm2 + 1, d.R2p));
     if (d.L1 == d.L2) d.TR1 = d.TR2 = std::max(d.TR1, d.TR2);
     // columns per block: as many as leave room for two CTAs on an SM, or for one
-    const size_t cap[2] = {113 * 1024, 226 * 1024};
+    const size_t cap[2] = {113 * 1024, DENSE_SMEM_MAX};
     for (int c = 0; c < 2; c++)
         for (int nb = 1; nb <= (d.K2 + 7) / 8; nb++) {
             d.NB = nb;
@@ -1903,8 +1905,8 @@ static cudaError_t launch_decon_dense(const DeconGeo &g, const DenseGeo &d, cons
     *launches = d.L1 != d.L2 ? 4 : 3;
     const size_t sp = dense_smem(d, d.hp1, d.hp2), sm = dense_smem(d, d.hm1, d.hm2);
     const void *fn = d.tiles == 1 ? (const void *)k_dense_window<1> : (const void *)k_dense_window<2>;
-    cudaError_t e = cudaFuncSetAttribute(k_dense_psf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sp);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    cudaError_t e = cudaFuncSetAttribute(k_dense_psf, cudaFuncAttributeMaxDynamicSharedMemorySize, DENSE_SMEM_MAX);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, DENSE_SMEM_MAX);
     if (e != cudaSuccess) return e;
     k_dense_psf<<<d.npsf, 2 * (sp + 1024) <= 227 * 1024 ? 256 : 512, sp, st>>>(g, d, psf, spec, smax, tabs);
     if (d.tiles == 1) k_dense_window<1><<<g.totalnum, d.nthr, sm, st>>>(g, d, mig, spec, smax, winout, tabs);
@@ -2784,7 +2786,7 @@ int swd_hilbert(swd_ctx *ctx, int nt, const float *rick, float *hrick)
 
 int swd_smooth(swd_ctx *ctx, int ntx, int ntz, int pml, int window, float *vp)
 {
-    if (!ctx || !vp || ntx <= 2 * pml || ntz <= 2 * pml || window < 0 || window > 64)
+    if (!ctx || !vp || ntx <= 2 * pml || ntz <= 2 * pml || window < 0 || window > SMOOTH_MAX_WINDOW)
         return fail(ctx, SWD_ERR_ARG, "bad smoothing arguments");
     CK(cudaSetDevice(ctx->dev));
     // normalised Gaussian of ini_model_mine (acoustic_HLVSPRTMC.cpp:1475-1501), built on the host
@@ -2809,8 +2811,9 @@ int swd_smooth(swd_ctx *ctx, int ntx, int ntz, int pml, int window, float *vp)
     CKR(to_dev(ctx, a.p, vp, sizeof(float) * n));
     CK(cudaMemcpyAsync(cf.p, coef.data(), sizeof(double) * coef.size(), cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemcpyAsync(b.p, a.p, sizeof(float) * n, cudaMemcpyDeviceToDevice, ctx->stream));
-    const size_t sm = sizeof(double) * (8 + 2 * (size_t)window) * (32 + 2 * (size_t)window);
-    CK(cudaFuncSetAttribute(k_smooth, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    const size_t sm = smooth_smem(window);
+    // the limit of every call: it belongs to the kernel, and another thread may be about to launch
+    CK(cudaFuncSetAttribute(k_smooth, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smooth_smem(SMOOTH_MAX_WINDOW)));
     k_smooth<<<dim3((ntz - 2 * pml + 31) / 32, (ntx - 2 * pml + 7) / 8), dim3(32, 8), sm, ctx->stream>>>(
         F(a), F(b), D(cf), ntx, ntz, pml, window);
     if (pml > 0) {
