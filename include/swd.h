@@ -250,7 +250,7 @@ int swd_rtm_batch(swd_ctx *ctx, int nshots, const swd_shot *shots, const float *
  *                 same results bit for bit. */
 #define SWD_OPT_LEAN 12
 /* SWD_OPT_RESIDENT 1 (default): passes of one wavefield or of a pair (modelling with its twin, RTM
- *                 with FP32 strips, batches at automatic size, Born modelling and the background of
+ *                 with FP32 strips, surveys of one or two shots, Born modelling and the background of
  *                 its adjoint from 8 steps per checkpoint on) on grids whose wavefields fit in the
  *                 SMs' shared memory and registers run as one cooperative launch that keeps the
  *                 fields on the chip between steps (stencil order 4, the other options at their

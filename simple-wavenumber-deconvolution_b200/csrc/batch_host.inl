@@ -61,7 +61,13 @@ static Wave batch_wave(swd_ctx *c, int k)
     return w;
 }
 
-// Whether both passes of a survey's shot run on the chip (resident.cuh), one shot at a time.
+// Surveys of at most this many shots run on the chip, one shot at a time.  Us per step and shot (nt
+// 400) of one / two / three / sixteen shots: batched by the step kernels 401 x 201 17.8 / 9.7 / 7.2 /
+// 5.3, 601 x 301 18.0 / 11.0 / 9.0 / 7.2, 801 x 401 19.8 / 14.7 / 13.0 / 11.9, 100 x 60 16.9 / 8.8 /
+// 6.0 / 2.4; on the chip, whatever their number, 9.6, 11.0, 13.9, 8.2.
+constexpr int BATCH_CHIP_SHOTS = 2;
+
+// Whether both passes of a survey's shot run on the chip (resident.cuh).
 static bool batch_resident(const swd_ctx *c, ResPlan *f, ResPlan *b)
 {
     return c->batch_opt == 0 && c->bwd_by_kind && c->image_blocks && c->strip_prec == SWD_STRIP_F32 &&
@@ -70,8 +76,8 @@ static bool batch_resident(const swd_ctx *c, ResPlan *f, ResPlan *b)
 
 // One batch: shots[idx[0..nb)].  probe_steps > 0 runs only that many forward and backward
 // steps and skips the per-shot post (autotuner probes; the stack is left alone).
-static int rtm_batch_run(swd_ctx *ctx, const swd_shot *shots, const float *const *ricks, const float *const *data,
-                         const int *idx, int nb, unsigned flags, int probe_steps)
+static int rtm_batch_once(swd_ctx *ctx, const swd_shot *shots, const float *const *ricks, const float *const *data,
+                          const int *idx, int nb, unsigned flags, int probe_steps)
 {
     std::vector<ShotPlan> P(nb);
     std::vector<ShotDesc> desc(nb);
@@ -271,6 +277,17 @@ static int rtm_batch_run(swd_ctx *ctx, const swd_shot *shots, const float *const
     return SWD_OK;
 }
 
+// The same, and again with the step kernels where an on-chip pass gave up (it has stacked nothing).
+static int rtm_batch_run(swd_ctx *ctx, const swd_shot *shots, const float *const *ricks, const float *const *data,
+                         const int *idx, int nb, unsigned flags, int probe_steps)
+{
+    CKR(rtm_batch_once(ctx, shots, ricks, data, idx, nb, flags, probe_steps));
+    if (!ctx->res_running) return SWD_OK;
+    CK(cudaStreamSynchronize(ctx->stream));
+    ctx->res_running = false;
+    return resident_failed(ctx) ? rtm_batch_once(ctx, shots, ricks, data, idx, nb, flags, probe_steps) : SWD_OK;
+}
+
 // Batch size by measurement: for B in 1, 2, 4, 8 (up to the number of shots and half the
 // free device memory), run a probe of 2 graph chunks forward and backward on the first B
 // shots twice and keep the B with the least time per shot of the second run.
@@ -326,21 +343,17 @@ int swd_rtm_batch(swd_ctx *ctx, int nshots, const swd_shot *shots, const float *
     std::vector<int> order(nshots);
     for (int i = 0; i < nshots; i++) order[i] = i;
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return shots[a].nt > shots[b].nt; });
-    int B = ctx->batch_opt;
-    ResPlan rf, rb;
+    // Surveys of one or two shots whose wavefields fit on the chip: one shot at a time there (while this
+    // call is the device's only one), without tuning the batch size, which larger surveys do for
+    // themselves.
     int done = 0;
-    if (batch_resident(ctx, &rf, &rb)) {
-        // one shot at a time; a pass that gave up has stacked nothing and runs again below
-        for (; done < nshots; done++) {
-            CKR(rtm_batch_run(ctx, shots, ricks, data, order.data() + done, 1, flags, 0));
-            CK(cudaStreamSynchronize(ctx->stream));
-            if (resident_failed(ctx)) break;
-        }
-        ctx->batch_tuned = 1;
-        B = 1;
-    }
-    if (B <= 0) {
-        if (ctx->batch_tuned <= 0) CKR(batch_autotune(ctx, shots, ricks, data, order.data(), nshots, flags, &ctx->batch_tuned));
+    ResPlan rf, rb;
+    while (nshots <= BATCH_CHIP_SHOTS && done < nshots && batch_resident(ctx, &rf, &rb))
+        CKR(rtm_batch_run(ctx, shots, ricks, data, order.data() + done++, 1, flags, 0));
+    int B = ctx->batch_opt;
+    if (B <= 0 && done < nshots) {
+        if (ctx->batch_tuned <= 0)
+            CKR(batch_autotune(ctx, shots, ricks, data, order.data() + done, nshots - done, flags, &ctx->batch_tuned));
         B = ctx->batch_tuned;
     }
     for (int g = done; g < nshots; g += B)

@@ -303,3 +303,40 @@ def test_on_chip_passes_after_a_device_reset(swd):
     own): the on-chip passes keep nothing from before."""
     r = subprocess.run([sys.executable, "-c", RESET, str(ROOT / "tests")], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stderr[-2000:]
+
+
+def test_surveys_keep_their_batches(swd):
+    """Surveys of one or two shots go on the chip and leave the batch size untuned; larger ones are tuned
+    and batched, also after an on-chip survey and with the on-chip passes switched off between; a last
+    shot left over from the batches may go on the chip, and give up there.  The stacks are the same bits."""
+    nt = 80
+    E, rng, (ntx, ntz) = _engine(swd, 100, 60, 10, nt, 6)
+    rick = swd.ricker_wave(nt, 60.0, 5e-4)
+    shots = [swd.ShotSpec(30 + 10 * k, 14, np.full(20, 70, np.int32), np.arange(20, 40).astype(np.int32), nt) for k in range(5)]
+    data = [rng.standard_normal((20, nt)).astype(np.float32) for _ in shots]
+
+    def stack(n):
+        E.stack_reset()
+        n0 = E.launch_count()
+        E.rtm_batch(shots[:n], [rick] * n, data[:n])
+        return E.stack(edge_zero=False), E.launch_count() - n0
+
+    E.set_option(swd.OPT_RESIDENT, 0)
+    E.set_option(swd.OPT_BATCH, 1)
+    ref = {n: stack(n) for n in (1, 2, 3, 5)}
+    E.set_option(swd.OPT_BATCH, 0)
+    E.set_option(swd.OPT_RESIDENT, 1)
+    for n in (1, 2):
+        got = stack(n)
+        assert np.array_equal(got[0], ref[n][0]) and got[1] < 0.2 * ref[n][1]
+    assert E.get_option(swd.OPT_BATCH_TUNED) == 0
+    E.set_option(swd.OPT_RESIDENT, 0)
+    assert np.array_equal(stack(5)[0], ref[5][0])
+    assert E.get_option(swd.OPT_BATCH_TUNED) == 4   # a batch of four takes about the time of one shot here
+    E.set_option(swd.OPT_RESIDENT, 1)
+    for n in (3, 5):
+        got = stack(n)
+        assert np.array_equal(got[0], ref[n][0]) and got[1] < 0.5 * ref[n][1]
+    E.set_option(swd.OPT_RESIDENT_STOP, 7)
+    assert np.array_equal(stack(5)[0], ref[5][0])
+    assert E.get_option(swd.OPT_RESIDENT) == 0
