@@ -2891,21 +2891,25 @@ int swd_decon(swd_ctx *ctx_in, const swd_decon_params *p, const float *migreal, 
         const bool dout = is_device_ptr_on(mig_dec, ctx->dev) && is_device_ptr_on(mig_coef, ctx->dev);
         DevBuf &bin = ctx->dcn[0], &bcoef = ctx->dcn[1], &bwin = ctx->dcn[2], &bout = ctx->dcn[3], &bws = ctx->dcn[4],
                &btab = ctx->dcn[5];
-        // the dense path where it applies and its scratch can be had, else the FFT windows
-        DenseGeo dg;
-        bool dense = dense_plan(g, dg);
-        if (dense && ensure(ctx, bws, sizeof(float) * dense_scratch(dg)) != SWD_OK) {
-            cudaGetLastError();
-            dense = false;
-        }
-        const int nblk = !dense && decon_persistent(g) ? decon_ws_blocks(g, ctx->dev) : 0;
-        if (!dense && decon_persistent(g) && nblk < 1) { rc = fail(ctx, SWD_ERR_CUDA, "decon: no launch shape for the window kernel"); break; }
-        if (!dense && decon_persistent(g)) rc = ensure(ctx, bws, sizeof(float) * (size_t)nblk * decon_ws_floats(g));
         if (!rc && !din) rc = ensure(ctx, bin, sizeof(float) * 2 * np);
         if (!rc) rc = ensure(ctx, bcoef, sizeof(float) * nout);
         if (!rc) rc = ensure(ctx, bwin, sizeof(float) * nout * g.totalnum);
         if (!rc) rc = ensure(ctx, btab, sizeof(float2) * decon_tab_len(g));
         if (!rc && !dout) rc = ensure(ctx, bout, sizeof(float) * 2 * np);
+        // the dense path where it applies and its scratch can be had beside what every path needs, else
+        // the FFT windows
+        DenseGeo dg;
+        bool dense = !rc && dense_plan(g, dg);
+        if (dense && ensure(ctx, bws, sizeof(float) * dense_scratch(dg)) != SWD_OK) {
+            cudaGetLastError();
+            dense = false;
+        }
+        int nblk = 0;
+        if (!rc && !dense && decon_persistent(g)) {
+            nblk = decon_ws_blocks(g, ctx->dev);
+            rc = nblk < 1 ? fail(ctx, SWD_ERR_CUDA, "decon: no launch shape for the window kernel")
+                          : ensure(ctx, bws, sizeof(float) * (size_t)nblk * decon_ws_floats(g));
+        }
         const float *im = din ? migreal : F(bin), *ps = din ? migpsf : F(bin) + np;
         float *od = dout ? mig_dec : F(bout), *oc = dout ? mig_coef : F(bout) + np;
         if (!rc && !din) rc = to_dev(ctx, bin.p, migreal, sizeof(float) * np);
