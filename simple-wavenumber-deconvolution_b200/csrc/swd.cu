@@ -133,6 +133,7 @@ struct swd_ctx {
     int use_resident = 1;         // SWD_OPT_RESIDENT
     int res_stop = 0;             // SWD_OPT_RESIDENT_STOP
     int use_march = 1;            // SWD_OPT_MARCH
+    bool in_smooth = false, in_decon = false, in_march = false;   // scratch in use (give_back)
     DevBuf marchl, marcht, marchr;   // strip blocks, tasks, ring of FP32 strips of a marching pass
     int nsm = 0, coop = 0;
     size_t smem_max = 0;
@@ -197,6 +198,44 @@ static int fail(swd_ctx *c, int code, const char *fmt, ...)
         if (r_ != SWD_OK) return r_;       \
     } while (0)
 
+static void drop(DevBuf &b)
+{
+    if (b.p) cudaFree(b.p);
+    b.p = nullptr;
+    b.n = 0;
+}
+
+// Scratch that only makes calls faster, given back when an allocation fails: the smoothing's buffers,
+// the deconvolution's workspace, a march's second copy of the field and strip ring (not while a call
+// uses them, nor the second copies that hold the fused path's fields).  Whether there was any.
+static bool give_back(swd_ctx *ctx)
+{
+    std::vector<DevBuf *> spare;
+    if (!ctx->in_smooth)
+        for (auto &b : ctx->smo) spare.push_back(&b);
+    if (!ctx->in_decon) spare.push_back(&ctx->dcn[4]);
+    const bool fields2 = ctx->path == SWD_PATH_FUSED || (ctx->kept.valid && ctx->kept.path == SWD_PATH_FUSED);
+    if (!ctx->in_march && !fields2) {
+        for (auto &b : ctx->wave2[0]) spare.push_back(&b);
+        spare.push_back(&ctx->marchr);
+    }
+    bool any = false;
+    for (DevBuf *b : spare) {
+        if (!b->p) continue;
+        if (!any) cudaStreamSynchronize(ctx->stream);
+        any = true;
+        drop(*b);
+    }
+    return any;
+}
+
+// marks scratch as in use for the time of a call
+struct InUse {
+    bool &flag;
+    explicit InUse(bool &f) : flag(f) { flag = true; }
+    ~InUse() { flag = false; }
+};
+
 static int ensure(swd_ctx *ctx, DevBuf &b, size_t bytes)
 {
     b.off = 0;
@@ -209,6 +248,10 @@ static int ensure(swd_ctx *ctx, DevBuf &b, size_t bytes)
     }
     if (bytes == 0) return SWD_OK;
     cudaError_t e = cudaMalloc(&b.p, bytes);
+    if (e == cudaErrorMemoryAllocation && give_back(ctx)) {
+        cudaGetLastError();
+        e = cudaMalloc(&b.p, bytes);
+    }
     if (e != cudaSuccess) {
         b.p = nullptr;
         return fail(ctx, SWD_ERR_ALLOC, "cudaMalloc(%zu bytes): %s", bytes, cudaGetErrorString(e));
@@ -1399,27 +1442,38 @@ static MWave march_wave(swd_ctx *c, int k, int in_par)
 
 // The march's own buffers, the second copy of the field and the ring of FP32 strips.  False, with the
 // memory given back, when they do not fit: the step kernels need neither.
-static bool march_room(swd_ctx *ctx, const FwdArgs &a)
+static bool march_room(swd_ctx *ctx, const FwdArgs &a, const std::vector<int4> &tasks, const std::vector<int> &list)
 {
-    bool ok = zero_wave2(ctx, 0) == SWD_OK;
+    bool ok = zero_wave2(ctx, 0) == SWD_OK && ensure(ctx, ctx->marcht, sizeof(int4) * tasks.size()) == SWD_OK &&
+              ensure(ctx, ctx->marchl, sizeof(int) * list.size()) == SWD_OK;
     if (ok && a.strips.buf && a.strips.prec)
         ok = ensure(ctx, ctx->marchr, sizeof(float) * (size_t)MARCH_RING * a.strips.slen) == SWD_OK;
     if (ok) return true;
     cudaGetLastError();
     cudaStreamSynchronize(ctx->stream);
-    auto drop = [](DevBuf &b) {
-        if (b.p) cudaFree(b.p);
-        b.p = nullptr;
-        b.n = 0;
-    };
     for (auto &b : ctx->wave2[0]) drop(b);
     drop(ctx->marchr);
     return false;
 }
 
-// One-wavefield forward pass by marches (after march_room); a holds the plain kernels' arguments.
-// The final state ends in wave[0].
-static int run_forward_march(swd_ctx *ctx, const FwdArgs &a, ShotPlan &P)
+// The 8-column, 128-row blocks of cell4's grid that hold strip cells: what k_march_encode runs over.
+static std::vector<int> march_strip_blocks(const swd_ctx *c)
+{
+    std::vector<int> list;
+    const dim3 grid = grid_blocks(c);
+    const int x1 = c->ntx - c->pmlc - 1, z1 = c->ntz - c->pmlc - 1, L = c->Lc, q = c->pmlc;
+    for (int by = 0; by < (int)grid.y; by++)
+        for (int bx = 0; bx < (int)grid.x; bx++) {
+            auto hit = [&](int xa, int xb, int za, int zb) { return by * 8 <= xb && by * 8 + 7 >= xa && bx * 128 <= zb && bx * 128 + 127 >= za; };
+            if (hit(q, x1, q, q + L - 1) || hit(q, x1, z1 - L + 1, z1) || hit(q, q + L - 1, q, z1) || hit(x1 - L + 1, x1, q, z1))
+                list.push_back(by * grid.x + bx);
+        }
+    return list;
+}
+
+// One-wavefield forward pass by marches; a holds the plain kernels' arguments.  The final state ends
+// in wave[0].  *ran is false when its buffers do not fit.
+static int run_forward_march(swd_ctx *ctx, const FwdArgs &a, ShotPlan &P, bool *ran)
 {
     MFwdArgs m;
     memset(&m, 0, sizeof m);
@@ -1427,36 +1481,29 @@ static int run_forward_march(swd_ctx *ctx, const FwdArgs &a, ShotPlan &P)
     m.wells = a.wells; m.seis = a.seis; m.nt = a.nt;
     std::vector<int4> tasks;
     march_tasks(ctx, tasks, a.seis ? P.wcol : std::vector<int>());
-    CKR(ensure(ctx, ctx->marcht, sizeof(int4) * tasks.size()));
+    const bool ring = a.strips.buf && a.strips.prec;
+    const std::vector<int> list = ring ? march_strip_blocks(ctx) : std::vector<int>();
+    const InUse mine(ctx->in_march);
+    *ran = march_room(ctx, a, tasks, list);
+    if (!*ran) return SWD_OK;
     CK(cudaMemcpyAsync(ctx->marcht.p, tasks.data(), sizeof(int4) * tasks.size(), cudaMemcpyHostToDevice, ctx->stream));
     m.task = (const int4 *)ctx->marcht.p;
     // strips: FP32 straight into the store, 16-bit codes by way of an FP32 ring encoded once per
     // captured chunk of steps
     static_assert(MARCH_RING == GRAPH_K, "the ring holds one chunk of steps");
-    const dim3 grid = grid_blocks(ctx);
     MEncodeArgs en;
     memset(&en, 0, sizeof en);
-    int nlist = 0;
-    if (a.strips.buf && a.strips.prec == 0) {
+    const int nlist = (int)list.size();
+    if (a.strips.buf && !ring) {
         m.strip = (float *)a.strips.buf;
         m.slen = a.strips.slen;
         m.ring = a.nt;
-    } else if (a.strips.buf) {
-        std::vector<int> list;
-        const int x1 = ctx->ntx - ctx->pmlc - 1, z1 = ctx->ntz - ctx->pmlc - 1, L = ctx->Lc, q = ctx->pmlc;
-        for (int by = 0; by < (int)grid.y; by++)
-            for (int bx = 0; bx < (int)grid.x; bx++) {
-                auto hit = [&](int xa, int xb, int za, int zb) { return by * 8 <= xb && by * 8 + 7 >= xa && bx * 128 <= zb && bx * 128 + 127 >= za; };
-                if (hit(q, x1, q, q + L - 1) || hit(q, x1, z1 - L + 1, z1) || hit(q, q + L - 1, q, z1) || hit(x1 - L + 1, x1, q, z1))
-                    list.push_back(by * grid.x + bx);
-            }
-        nlist = (int)list.size();
-        CKR(ensure(ctx, ctx->marchl, sizeof(int) * nlist));
+    } else if (ring) {
         CK(cudaMemcpyAsync(ctx->marchl.p, list.data(), sizeof(int) * nlist, cudaMemcpyHostToDevice, ctx->stream));
         m.strip = F(ctx->marchr);
         m.slen = a.strips.slen;
         m.ring = MARCH_RING;
-        en.g = a.g; en.ringbuf = m.strip; en.itp = a.itp; en.strips = a.strips; en.list = I32(ctx->marchl); en.gx = grid.x;
+        en.g = a.g; en.ringbuf = m.strip; en.itp = a.itp; en.strips = a.strips; en.list = I32(ctx->marchl); en.gx = grid_blocks(ctx).x;
     }
     m.w = march_wave(ctx, 0, 0);
     const int nwarp = (int)tasks.size();
@@ -1596,8 +1643,11 @@ static int run_forward(swd_ctx *ctx, FwdJob &J, ShotPlan &P)
         CKR(run_resident(ctx, r, rp, a.s0_out ? 3 : 0, &ran));
         if (ran) return SWD_OK;
     }
-    if (nw == 1 && !a.ck.every && !a.ds.buf && !a.s0_out && !a.dkappa && !a.dck && march_ok(ctx) && march_room(ctx, a))
-        return run_forward_march(ctx, a, P);
+    if (nw == 1 && !a.ck.every && !a.ds.buf && !a.s0_out && !a.dkappa && !a.dck && march_ok(ctx)) {
+        bool ran;
+        CKR(run_forward_march(ctx, a, P, &ran));
+        if (ran) return SWD_OK;
+    }
     // one wavefield without checkpoints: the velocity kernel with TMA-staged pressure
     // the plain single-wavefield forward (RTM forward, modelling without a twin): variants of the
     // velocity and pressure launches, chosen by the tuner when SWD_OPT_AUTOTUNE is on
@@ -2805,6 +2855,7 @@ int swd_smooth(swd_ctx *ctx, int ntx, int ntz, int pml, int window, float *vp)
     const size_t n = (size_t)ntx * ntz;
     // scratch kept by the context: three allocations and releases cost more than the smoothing
     DevBuf &a = ctx->smo[0], &b = ctx->smo[1], &cf = ctx->smo[2];
+    const InUse mine(ctx->in_smooth);
     CKR(ensure(ctx, a, sizeof(float) * n));
     CKR(ensure(ctx, b, sizeof(float) * n));
     CKR(ensure(ctx, cf, sizeof(double) * coef.size()));
@@ -2899,6 +2950,7 @@ int swd_decon(swd_ctx *ctx_in, const swd_decon_params *p, const float *migreal, 
         // the dense path where it applies and its scratch can be had beside what every path needs, else
         // the FFT windows
         DenseGeo dg;
+        const InUse ws(ctx->in_decon);
         bool dense = !rc && dense_plan(g, dg);
         if (dense && ensure(ctx, bws, sizeof(float) * dense_scratch(dg)) != SWD_OK) {
             cudaGetLastError();

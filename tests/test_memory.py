@@ -65,3 +65,85 @@ def test_decon_falls_back_to_the_fft_windows(swd):
     assert not np.array_equal(got, ref)                 # the other path
     assert rel_l2(got, ref) < 2e-5                      # (single-precision roundings of both, as between them elsewhere)
     assert np.array_equal(job(E), ref)                  # and back, with the memory back
+
+
+class Rtm:
+    """One shot on a grid whose forward pass takes a second copy of the field (94 MB)."""
+
+    nt = 66
+
+    def __init__(self, swd):
+        nx, nz, pml = 3001, 1509, 13
+        rng = np.random.default_rng(3)
+        self.swd, p = swd, pml + 4
+        self.vp = swd.pad_model((1900.0 + 900.0 * np.arange(nz)[None, :] / nz + rng.uniform(-80, 80, (nx, 1))).astype(np.float32), p)
+        self.rho = np.full_like(self.vp, 1000.0)
+        self.dims = (nx, nz, pml, 4, 5.0, 5.0, 5e-4, self.nt)
+        self.shot = swd.ShotSpec(p + nx // 2, p + 4, np.full(40, p + nx // 2 + 5, np.int32), (p + np.arange(40)).astype(np.int32), self.nt)
+        self.rick = swd.ricker_wave(self.nt, 60.0, 5e-4)
+        self.data = rng.standard_normal((40, self.nt)).astype(np.float32)
+
+    def engine(self):
+        E = self.swd.Engine(*self.dims)
+        E.setup_default(self.vp, self.rho)
+        return E
+
+    def backward(self, E):
+        E.rtm_backward(self.shot, self.data, flags=self.swd.RTM_NO_STACK, want=())
+        return E.rtm_raw()[:2]
+
+    def steps(self, E):
+        """The shot by the step kernels (no second copy)."""
+        E.set_option(self.swd.OPT_MARCH, 0)
+        E.rtm_forward(self.shot, self.rick)
+        return self.backward(E)
+
+
+@pytest.mark.parametrize("first", ["march", "smooth", "decon"])
+def test_scratch_of_an_earlier_call_is_given_back(swd, first):
+    """The second call needs more than is left on the device, but no more than with the scratch of the
+    first (94 to 160 MB) given back."""
+    job = Rtm(swd)
+    other = Decon(swd) if first == "decon" else None
+    big = np.full((5000, 4000), 2000.0, np.float32)
+
+    def begin(E):
+        if first == "march":
+            E.rtm_forward(job.shot, job.rick)
+        elif first == "smooth":
+            E.smooth(big, 17, 2)
+        else:
+            other(E)
+
+    end = job.backward if first == "march" else job.steps
+    E = job.engine()
+    begin(E)
+    n0 = E.device_bytes()
+    ref = end(E)
+    need = E.device_bytes() - n0
+    E.close()
+    E = job.engine()
+    begin(E)
+    with Filled(need - 20 * MB):
+        got = end(E)
+    for a, b in zip(got, ref):
+        assert np.abs(b).max() > 0 and np.array_equal(a, b)
+
+
+def test_march_without_room_for_its_second_copy(swd):
+    job = Rtm(swd)
+    E = job.engine()
+    E.set_option(swd.OPT_MARCH, 0)
+    n0 = E.device_bytes()
+    ref = E.forward(job.shot, job.rick)
+    need = E.device_bytes() - n0
+    E.close()
+    E = job.engine()
+    with Filled(need + 45 * MB):
+        n0 = E.launch_count()
+        got = E.forward(job.shot, job.rick)
+        assert E.launch_count() - n0 >= 2 * job.nt
+    assert np.abs(ref).max() > 0 and np.array_equal(got, ref)
+    n0 = E.launch_count()
+    assert np.array_equal(E.forward(job.shot, job.rick), ref)
+    assert E.launch_count() - n0 < 2 * job.nt
