@@ -1322,28 +1322,34 @@ static bool resident_plan(const swd_ctx *c, int nw, ResPlan *plan, bool born = f
     return res_plan(c->ntx, c->ntz, c->pmlc, c->nsm, c->smem_max, nw, born, plan);
 }
 
-// One pass of a.nsteps steps from a.t0.  *ran is false when the launch was refused (fewer SMs than
-// the device reports, say): the caller goes on with the plain kernels.  An error word that a kernel sets (a wait that gave up)
-// makes later launches return at once; resident_failed reads it after the stream has drained.
+// Exchange words and error words of the on-chip passes; false when they cannot be had.
+static bool resident_room(swd_ctx *ctx, const ResPlan &p)
+{
+    const bool fresh = ctx->resll.n < p.ll_bytes || !ctx->resll.p || ctx->res_epoch > 0x7f000000u;
+    void *h = nullptr;
+    bool ok = ensure(ctx, ctx->resll, p.ll_bytes) == SWD_OK;
+    if (ok && fresh) {   // no stale word may carry a tag to come
+        ok = cudaMemsetAsync(ctx->resll.p, 0, ctx->resll.n, ctx->stream) == cudaSuccess;
+        ctx->res_epoch = 0;
+    }
+    if (ok && !ctx->reserr.p)
+        ok = ensure(ctx, ctx->reserr, 64) == SWD_OK && cudaMemsetAsync(ctx->reserr.p, 0, 64, ctx->stream) == cudaSuccess;
+    if (ok && !ctx->res_flag) {
+        ok = cudaHostAlloc(&h, 64, cudaHostAllocMapped) == cudaSuccess;
+        if (ok) ctx->res_flag = (volatile int *)memset(h, 0, 64);
+    }
+    if (!ok) cudaGetLastError();
+    return ok;
+}
+
+// One pass of a.nsteps steps from a.t0.  *ran is false when its buffers do not fit or the launch was
+// refused (fewer SMs than the device reports, say): the caller goes on with the plain kernels.  An
+// error word that a kernel sets (a wait that gave up) makes later launches return at once;
+// resident_failed reads it after the stream has drained.
 static int run_resident(swd_ctx *ctx, ResArgs &a, const ResPlan &p, int mode, bool *ran)
 {
     *ran = false;
-    const bool fresh = ctx->resll.n < p.ll_bytes || !ctx->resll.p || ctx->res_epoch > 0x7f000000u;
-    CKR(ensure(ctx, ctx->resll, p.ll_bytes));
-    if (fresh) {   // no stale word may carry a tag to come
-        CK(cudaMemsetAsync(ctx->resll.p, 0, ctx->resll.n, ctx->stream));
-        ctx->res_epoch = 0;
-    }
-    if (!ctx->reserr.p) {
-        CKR(ensure(ctx, ctx->reserr, 64));
-        CK(cudaMemsetAsync(ctx->reserr.p, 0, 64, ctx->stream));
-    }
-    if (!ctx->res_flag) {
-        void *h = nullptr;
-        CK(cudaHostAlloc(&h, 64, cudaHostAllocMapped));
-        memset(h, 0, 64);
-        ctx->res_flag = (volatile int *)h;
-    }
+    if (!resident_room(ctx, p)) return SWD_OK;
     void *hd = nullptr;
     CK(cudaHostGetDevicePointer(&hd, (void *)ctx->res_flag, 0));
     a.ll = (uint4 *)ctx->resll.p;

@@ -147,3 +147,30 @@ def test_march_without_room_for_its_second_copy(swd):
     n0 = E.launch_count()
     assert np.array_equal(E.forward(job.shot, job.rick), ref)
     assert E.launch_count() - n0 < 2 * job.nt
+
+
+def test_on_chip_pass_without_room_for_its_exchange_words(swd):
+    """Every buffer of the step kernels is there, and not two megabytes more."""
+    drv = C.CDLL("libcuda.so.1")
+    nt = 60
+    E = swd.Engine(401, 201, 10, 4, 5.0, 5.0, 5e-4, nt)
+    vp = np.full((429, 229), 2000.0, np.float32)
+    E.setup_default(vp, np.full_like(vp, 1000.0))
+    s = swd.ShotSpec(60, 16, np.full(20, 70, np.int32), np.arange(20, 40).astype(np.int32), nt)
+    rick = swd.ricker_wave(nt, 60.0, 5e-4)
+    E.set_option(swd.OPT_RESIDENT, 0)
+    ref = E.forward(s, rick)
+    E.set_option(swd.OPT_RESIDENT, 1)
+    taken = []
+    with Filled(64 * MB):
+        for n in (16, 8, 4, 2):
+            p = C.c_uint64()
+            while len(taken) < 100 and drv.cuMemAlloc_v2(C.byref(p), C.c_size_t(n * MB)) == 0:
+                taken.append(p.value)
+        got = E.forward(s, rick)
+        for p in taken:
+            assert drv.cuMemFree_v2(C.c_uint64(p)) == 0
+    assert np.abs(ref).max() > 0 and np.array_equal(got, ref)
+    n0 = E.launch_count()
+    assert np.array_equal(E.forward(s, rick), ref)
+    assert E.launch_count() - n0 < nt                   # on the chip again
