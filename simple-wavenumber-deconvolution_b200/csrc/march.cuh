@@ -139,7 +139,7 @@ struct MFwdArgs {
     const float *wav0;
     int sx, sz;
     // boundary strips in FP32: the store itself ([nt][slen]), or a ring of MARCH_RING steps that
-    // k_march_encode turns into 16-bit codes; nullptr to skip
+    // k_march_encode turns into 16-bit codes; nullptr to skip (ring then 1)
     float *strip;
     int slen, ring;
     Wells wells;

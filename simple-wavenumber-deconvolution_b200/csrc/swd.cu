@@ -1485,6 +1485,7 @@ static int run_forward_march(swd_ctx *ctx, const FwdArgs &a, ShotPlan &P, bool *
     memset(&m, 0, sizeof m);
     m.g = a.g; m.c = a.c; m.m = a.m; m.itp = a.itp; m.wav0 = a.wav0; m.sx = a.sx; m.sz = a.sz;
     m.wells = a.wells; m.seis = a.seis; m.nt = a.nt;
+    m.ring = 1;   // without strips: steps are taken modulo it
     std::vector<int4> tasks;
     march_tasks(ctx, tasks, a.seis ? P.wcol : std::vector<int>());
     const bool ring = a.strips.buf && a.strips.prec;
