@@ -1920,7 +1920,8 @@ static bool dense_plan(const DeconGeo &g, DenseGeo &d)
     d.TR1 = up8(std::max(d.hm1 + 1, d.R1p));
     d.TR2 = up8(std::max(d.hm2 + 1, d.R2p));
     if (d.L1 == d.L2) d.TR1 = d.TR2 = std::max(d.TR1, d.TR2);
-    // columns per block: as many as leave room for two CTAs on an SM, or for one
+    // columns per block: as many as leave room for two CTAs on an SM, or for one.  Two CTAs take blocks
+    // of 16 columns or more, or the eight that are all of a transform of up to 15 points
     const size_t cap[2] = {113 * 1024, DENSE_SMEM_MAX};
     for (int c = 0; c < 2; c++)
         for (int nb = 1; nb <= (d.K2 + 7) / 8; nb++) {
@@ -1930,7 +1931,7 @@ static bool dense_plan(const DeconGeo &g, DenseGeo &d)
             d.yp = odd4(d.blk);
             d.KT1 = odd4(std::max(d.K1p, d.L1 == d.L2 ? nb * d.blk : 0));
             d.KT2 = d.L1 == d.L2 ? d.KT1 : odd4(nb * d.blk);
-            if (dense_smem(d, d.hm1, d.hm2) > cap[c] || (c == 0 && d.blk < 16)) continue;
+            if (dense_smem(d, d.hm1, d.hm2) > cap[c] || (c == 0 && d.blk < 16 && nb > 1)) continue;
             const int tiles = 4 * (d.R1p / 4) * (d.R2p / 8);
             d.nthr = c == 0 ? 256 : 512;
             d.tiles = 1;
