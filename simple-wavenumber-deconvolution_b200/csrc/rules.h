@@ -1,6 +1,7 @@
 // rules.h -- sizes for which the engine takes one kernel path or another: plain host functions of
 // numbers, without CUDA, so that they can be checked over whole ranges of sizes on the CPU.
 #pragma once
+#include <cstddef>
 
 namespace swd {
 
@@ -14,5 +15,15 @@ inline bool strip_bands_apart(int ntz, int pmlc, int Lc) { return ntz - 2 * pmlc
 // one multiply-add per array).  Grids beyond that keep the step kernels: two copies of the field and
 // six more arrays of 2^31 cells leave no room on a device of 180 GB for anything else.
 inline bool march_index_fits(int ntx, int ldz) { return (long long)ntx * ldz <= 0x7fffffffLL; }
+
+// Whether a smoothing window of this half width works on a tile of doubles in shared memory, on a grid
+// of so many blocks (32 x 8 cells).  Wider windows leave an SM fewer blocks and so too few warps for the
+// additions' latency, first where the grid is one wave or little more.  Call with the tile / taps from
+// memory, us, at half widths 24 / 28 / 32 / 40 / 48: 1669 x 869 (5,500 blocks) 1628 / 2272 / 2984 / 5656 /
+// 8881 and 1729 / 2311 / 2978 / 4570 / 6500; 600 x 400 (860 blocks) 312 / 616 / 655 / 1028 / 1506 and
+// 344 / 449 / 566 / 861 / 1221.
+constexpr int SMOOTH_TILE_WINDOW = 32;
+inline bool smooth_tile(int window, long long blocks) { return window <= 24 || (window <= SMOOTH_TILE_WINDOW && blocks >= 4000); }
+inline size_t smooth_smem(int w) { return sizeof(double) * (8 + 2 * (size_t)w) * (32 + 2 * (size_t)w); }
 
 }  // namespace swd

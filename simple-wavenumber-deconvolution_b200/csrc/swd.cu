@@ -674,28 +674,37 @@ __global__ void k_stack_out(const double *__restrict__ st, float *out, int nx, i
 
 // Gaussian smoothing of ini_model_mine (acoustic_HLVSPRTMC.cpp:1514-1556): double
 // accumulation in the reference's loop order with unfused multiply and add, clamped
-// indices, rows iz < pml+8 unchanged.  Coefficients come from the host.  The block's cells and
-// their window are converted to double once, in shared memory (8 + 2w columns of 32 + 2w rows):
-// converting at every tap kept the conversion unit busy (1669 x 869, 11 x 11 window: 120 -> 83 us).
-constexpr int SMOOTH_MAX_WINDOW = 64;
-static size_t smooth_smem(int w) { return sizeof(double) * (8 + 2 * (size_t)w) * (32 + 2 * (size_t)w); }
+// indices, rows iz < pml+8 unchanged.  Coefficients come from the host.
+//
+// TILE: the block's cells and their window are converted to double once, in shared memory (8 + 2w
+// columns of 32 + 2w rows): converting at every tap kept the conversion unit busy (1669 x 869, 11 x 11
+// window: 120 -> 83 us).  Wider windows (smooth_tile) read their taps from memory: the tile would leave
+// an SM too few warps.
+template <bool TILE>
 __global__ void __launch_bounds__(256) k_smooth(const float *__restrict__ vin, float *vout, const double *__restrict__ coef, int ntx,
                                                 int ntz, int pml, int w)
 {
     extern __shared__ double sv[];
     const int z0 = blockIdx.x * 32 + pml, x0 = blockIdx.y * 8 + pml, nr = 32 + 2 * w, nc = 8 + 2 * w;
-    for (int c = threadIdx.y; c < nc; c += 8) {
-        const int x = min(max(x0 - w + c, 0), ntx - 1);
-        for (int r = threadIdx.x; r < nr; r += 32) sv[c * nr + r] = (double)vin[(size_t)x * ntz + min(max(z0 - w + r, 0), ntz - 1)];
+    if (TILE) {
+        for (int c = threadIdx.y; c < nc; c += 8) {
+            const int x = min(max(x0 - w + c, 0), ntx - 1);
+            for (int r = threadIdx.x; r < nr; r += 32) sv[c * nr + r] = (double)vin[(size_t)x * ntz + min(max(z0 - w + r, 0), ntz - 1)];
+        }
+        __syncthreads();
     }
-    __syncthreads();
     const int iz = z0 + threadIdx.x, ix = x0 + threadIdx.y;
     if (iz > ntz - pml - 1 || ix > ntx - pml - 1) return;
     const int wx = 2 * w + 1;
     const double *v = sv + threadIdx.y * nr + threadIdx.x;   // the window's first cell
     double s = 0.0;
-    for (int a = 0; a < wx; a++)
-        for (int b = 0; b < wx; b++) s = __dadd_rn(s, __dmul_rn(v[b * nr + a], __ldg(coef + a * wx + b)));
+    for (int a = 0; a < wx; a++) {
+        const int z = min(max(iz - w + a, 0), ntz - 1);
+        for (int b = 0; b < wx; b++) {
+            const double t = TILE ? v[b * nr + a] : (double)vin[(size_t)min(max(ix - w + b, 0), ntx - 1) * ntz + z];
+            s = __dadd_rn(s, __dmul_rn(t, __ldg(coef + a * wx + b)));
+        }
+    }
     const size_t ip = (size_t)ix * ntz + iz;
     vout[ip] = iz < pml + 8 ? vin[ip] : (float)s;
 }
@@ -2844,7 +2853,7 @@ int swd_hilbert(swd_ctx *ctx, int nt, const float *rick, float *hrick)
 
 int swd_smooth(swd_ctx *ctx, int ntx, int ntz, int pml, int window, float *vp)
 {
-    if (!ctx || !vp || ntx <= 2 * pml || ntz <= 2 * pml || window < 0 || window > SMOOTH_MAX_WINDOW)
+    if (!ctx || !vp || ntx <= 2 * pml || ntz <= 2 * pml || window < 0 || window > 64)
         return fail(ctx, SWD_ERR_ARG, "bad smoothing arguments");
     CK(cudaSetDevice(ctx->dev));
     // normalised Gaussian of ini_model_mine (acoustic_HLVSPRTMC.cpp:1475-1501), built on the host
@@ -2870,11 +2879,14 @@ int swd_smooth(swd_ctx *ctx, int ntx, int ntz, int pml, int window, float *vp)
     CKR(to_dev(ctx, a.p, vp, sizeof(float) * n));
     CK(cudaMemcpyAsync(cf.p, coef.data(), sizeof(double) * coef.size(), cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemcpyAsync(b.p, a.p, sizeof(float) * n, cudaMemcpyDeviceToDevice, ctx->stream));
-    const size_t sm = smooth_smem(window);
-    // the limit of every call: it belongs to the kernel, and another thread may be about to launch
-    CK(cudaFuncSetAttribute(k_smooth, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smooth_smem(SMOOTH_MAX_WINDOW)));
-    k_smooth<<<dim3((ntz - 2 * pml + 31) / 32, (ntx - 2 * pml + 7) / 8), dim3(32, 8), sm, ctx->stream>>>(
-        F(a), F(b), D(cf), ntx, ntz, pml, window);
+    const dim3 grid((ntz - 2 * pml + 31) / 32, (ntx - 2 * pml + 7) / 8), block(32, 8);
+    if (smooth_tile(window, (long long)grid.x * grid.y)) {
+        // the limit of every call: it belongs to the kernel, and another thread may be about to launch
+        CK(cudaFuncSetAttribute(k_smooth<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smooth_smem(SMOOTH_TILE_WINDOW)));
+        k_smooth<true><<<grid, block, smooth_smem(window), ctx->stream>>>(F(a), F(b), D(cf), ntx, ntz, pml, window);
+    } else {
+        k_smooth<false><<<grid, block, 0, ctx->stream>>>(F(a), F(b), D(cf), ntx, ntz, pml, window);
+    }
     if (pml > 0) {
         k_pml_x<<<dim3((ntz - 2 * pml + 127) / 128, 2 * pml), 128, 0, ctx->stream>>>(F(b), ntx, ntz, pml);
         k_pml_z<<<(unsigned)(((size_t)ntx * 2 * pml + 127) / 128), 128, 0, ctx->stream>>>(F(b), ntx, ntz, pml);

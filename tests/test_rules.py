@@ -10,6 +10,8 @@ WRAP = """
 #include "rules.h"
 extern "C" {
 int bands_apart(int ntz, int pmlc, int Lc) { return swd::strip_bands_apart(ntz, pmlc, Lc); }
+int smooth_tile(int window, long long blocks) { return swd::smooth_tile(window, blocks); }
+long long smooth_smem(int window) { return swd::smooth_smem(window); }
 int index_fits(int ntx, int ldz) { return swd::march_index_fits(ntx, ldz); }
 }
 """
@@ -56,3 +58,15 @@ def test_march_index_range(rules):
         for ntx in (100, 4069, (2 ** 31 - 1) // ldz, (2 ** 31 - 1) // ldz + 1, 46341, 2 ** 31 // ldz + 100):
             fits = (ntx - 1) * ldz + ldz - 4 < 2 ** 31 and ntx * ldz < 2 ** 31
             assert bool(rules.index_fits(ntx, ldz)) == fits, (ntx, ldz)
+
+
+def test_smoothing_tiles_leave_room_for_warps(rules):
+    """Wherever a tile is used an SM holds at least four blocks of it (227 KB, 1 KB each reserved), six on
+    grids of few blocks; the reference's window always uses it."""
+    rules.smooth_tile.argtypes, rules.smooth_smem.restype = [C.c_int, C.c_longlong], C.c_longlong
+    assert rules.smooth_tile(5, 1)
+    for blocks in (1, 500, 3999, 4000, 10 ** 9):
+        for w in range(65):
+            per_sm = 227 * 1024 // (rules.smooth_smem(w) + 1024)
+            if rules.smooth_tile(w, blocks):
+                assert per_sm >= (4 if blocks >= 4000 else 6), (w, blocks)
