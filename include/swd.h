@@ -259,7 +259,7 @@ int swd_rtm_batch(swd_ctx *ctx, int nshots, const swd_shot *shots, const float *
 /* SWD_OPT_MARCH 1 (default): on grids whose fields fill the device's L2, the forward passes of one
  *                 wavefield (RTM, modelling without a twin) run each time step as one sweep along x
  *                 that makes both half steps (stencil order 4, the other options at their defaults,
- *                 no profiling).  The same results bit for bit.  0: the step kernels. */
+ *                 no profiling, an absorbing frame that is not most of the grid).  The same results bit for bit.  0: the step kernels. */
 #define SWD_OPT_MARCH 14
 /* SWD_OPT_RESIDENT_STOP n (default 0: off), for tests of the recovery from an on-chip pass in which a
  *                 wait for a neighbouring tile gave up (after a second or two): n > 0 ends the passes

@@ -16,6 +16,14 @@ inline bool strip_bands_apart(int ntz, int pmlc, int Lc) { return ntz - 2 * pmlc
 // six more arrays of 2^31 cells leave no room on a device of 180 GB for anything else.
 inline bool march_index_fits(int ntx, int ldz) { return (long long)ntx * ldz <= 0x7fffffffLL; }
 
+// Whether a march pays on a grid of so many cells: the tasks that touch the frame (17 columns and 7 more
+// to fill the windows, 128 rows of which 112 are their own) may work on no more cells than the grid
+// has.  Flat or narrow grids and wide frames have more of them, at twice the instructions each.  Forward
+// step with 16-bit strips, us, march / step kernels, with that work as a share of the grid: 4001 x 1601
+// 0.26 54.2 / 62.8, 2300 x 2300 with a 200-cell frame 0.56 65.1 / 67.2, 12000 x 500 0.97 74.0 / 72.0,
+// 16000 x 400 1.17 92.1 / 81.4, 20000 x 300 1.48 106.2 / 84.1, 40000 x 160 2.38 184.7 / 125.1.
+inline bool march_pays(size_t frame_tasks, long long cells) { return (long long)frame_tasks * (17 + 7) * 128 <= cells; }
+
 // Whether a smoothing window of this half width works on a tile of doubles in shared memory, on a grid
 // of so many blocks (32 x 8 cells).  Wider windows leave an SM fewer blocks and so too few warps for the
 // additions' latency, first where the grid is one wave or little more.  Call with the tile / taps from

@@ -133,6 +133,7 @@ struct swd_ctx {
     int use_resident = 1;         // SWD_OPT_RESIDENT
     int res_stop = 0;             // SWD_OPT_RESIDENT_STOP
     int use_march = 1;            // SWD_OPT_MARCH
+    int march_pay = -1;           // march_pays for this grid and frame, -1: not looked at yet
     bool in_smooth = false, in_decon = false, in_march = false;   // scratch in use (give_back)
     DevBuf marchl, marcht, marchr;   // strip blocks, tasks, ring of FP32 strips of a marching pass
     int nsm = 0, coop = 0;
@@ -1433,14 +1434,16 @@ static void march_tasks_of(const swd_ctx *c, std::vector<int4> &t, int wide, int
 // fewer columns twice, but a warp by itself issues one instruction in six cycles); frame tasks
 // MARCH_NARROW.  Forward step, us, at 57 / 49 / 41 / 33 columns: 4001 x 1601 53.0 / 53.8 / 54.6 /
 // 57.7, 3301 x 1501 43.1 / - / 40.4 / 42.8, 3001 x 1403 38.5 / - / 35.7 / 34.1.
-static void march_tasks(const swd_ctx *c, std::vector<int4> &t, const std::vector<int> &wcol)
+// Returns the number of frame tasks.
+static size_t march_tasks(const swd_ctx *c, std::vector<int4> &t, const std::vector<int> &wcol)
 {
+    size_t n = 0;
     for (int wide = 57; wide >= 33; wide -= 8) {
-        size_t n = 0;
         t.clear();
         march_tasks_of(c, t, wide, MARCH_NARROW, wcol, &n);
-        if (n >= (size_t)6 * std::max(c->nsm, 1)) return;
+        if (n >= (size_t)6 * std::max(c->nsm, 1)) break;
     }
+    return t.size() - n;
 }
 
 static MWave march_wave(swd_ctx *c, int k, int in_par)
@@ -1487,16 +1490,21 @@ static std::vector<int> march_strip_blocks(const swd_ctx *c)
 }
 
 // One-wavefield forward pass by marches; a holds the plain kernels' arguments.  The final state ends
-// in wave[0].  *ran is false when its buffers do not fit.
+// in wave[0].  *ran is false when its buffers do not fit or the frame is too much of the grid.
 static int run_forward_march(swd_ctx *ctx, const FwdArgs &a, ShotPlan &P, bool *ran)
 {
+    *ran = false;
+    if (ctx->march_pay == 0) return SWD_OK;
     MFwdArgs m;
     memset(&m, 0, sizeof m);
     m.g = a.g; m.c = a.c; m.m = a.m; m.itp = a.itp; m.wav0 = a.wav0; m.sx = a.sx; m.sz = a.sz;
     m.wells = a.wells; m.seis = a.seis; m.nt = a.nt;
     m.ring = 1;   // without strips: steps are taken modulo it
     std::vector<int4> tasks;
-    march_tasks(ctx, tasks, a.seis ? P.wcol : std::vector<int>());
+    static_assert(MARCH_NARROW == 17 && MARCH_OWN == 112, "the sizes march_pays speaks of");
+    const size_t frame = march_tasks(ctx, tasks, a.seis ? P.wcol : std::vector<int>());
+    ctx->march_pay = march_pays(frame, (long long)ctx->ntx * ctx->ntz);
+    if (!ctx->march_pay) return SWD_OK;
     const bool ring = a.strips.buf && a.strips.prec;
     const std::vector<int> list = ring ? march_strip_blocks(ctx) : std::vector<int>();
     const InUse mine(ctx->in_march);
@@ -2183,6 +2191,7 @@ int swd_set_cpml(swd_ctx *ctx, const float *a_x, const float *a_x_half, const fl
     };
     span(a_x, a_x_half, ctx->ntx, ctx->lean);
     span(a_z, a_z_half, ctx->ntz, ctx->lean + 2);
+    ctx->march_pay = -1;
     return SWD_OK;
 }
 

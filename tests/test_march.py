@@ -66,3 +66,15 @@ def test_march_needs_a_large_grid(swd):
         n0 = E.launch_count()
         E.rtm_forward(s, swd.ricker_wave(nt, 25.0, 5e-4))
         assert E.launch_count() - n0 >= 2 * nt
+
+
+def test_flat_grid_keeps_the_step_kernels(swd):
+    """A large grid that is nearly all frame: the march would take 1.6 times as long."""
+    nx, nz, pml, nt = 36000, 100, 10, 64
+    E = swd.Engine(nx, nz, pml, 4, 5.0, 5.0, 5e-4, nt)
+    vp = np.full((nx + 28, nz + 28), 2000.0, np.float32)
+    E.setup_default(vp, np.full_like(vp, 1000.0))
+    s = swd.ShotSpec(60, 60, np.array([70], np.int32), np.array([60], np.int32), nt)
+    n0 = E.launch_count()
+    E.forward(s, swd.ricker_wave(nt, 25.0, 5e-4))
+    assert E.launch_count() - n0 >= 2 * nt

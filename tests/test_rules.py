@@ -10,6 +10,7 @@ WRAP = """
 #include "rules.h"
 extern "C" {
 int bands_apart(int ntz, int pmlc, int Lc) { return swd::strip_bands_apart(ntz, pmlc, Lc); }
+int march_pays(size_t frame_tasks, long long cells) { return swd::march_pays(frame_tasks, cells); }
 int smooth_tile(int window, long long blocks) { return swd::smooth_tile(window, blocks); }
 long long smooth_smem(int window) { return swd::smooth_smem(window); }
 int index_fits(int ntx, int ldz) { return swd::march_index_fits(ntx, ldz); }
@@ -70,3 +71,26 @@ def test_smoothing_tiles_leave_room_for_warps(rules):
             per_sm = 227 * 1024 // (rules.smooth_smem(w) + 1024)
             if rules.smooth_tile(w, blocks):
                 assert per_sm >= (4 if blocks >= 4000 else 6), (w, blocks)
+
+
+def test_march_wants_little_frame(rules):
+    """Frame tasks counted as the launch cuts them (row tiles of 112, frame chunks of 17 columns, lean
+    chunks of 33 or more): squarish grids march, flat and narrow ones keep the step kernels."""
+    rules.march_pays.argtypes = [C.c_size_t, C.c_longlong]
+
+    def pays(nx, nz, pml, wide):
+        p = pml + 4
+        ntx, ntz = nx + 2 * p, nz + 2 * p
+        frame = 0
+        for bz in range(-(-ntz // 112)):
+            x, zl = 0, bz * 112 - 8 >= p + 4 and bz * 112 + 120 <= ntz - p - 4
+            while x < ntx:
+                lean = zl and x - 8 >= p + 4 and x + wide + 8 <= ntx - p - 4
+                frame += not lean
+                x += wide if lean else 17
+        return bool(rules.march_pays(frame, ntx * ntz))
+
+    for grid in ((4001, 1601, 30, 57), (3001, 1403, 30, 33), (2400, 2400, 100, 49), (12000, 500, 30, 33), (400, 15000, 30, 49)):
+        assert pays(*grid), grid
+    for grid in ((16000, 400, 30, 33), (30000, 200, 10, 33), (60000, 100, 10, 33), (60, 90000, 10, 33)):
+        assert not pays(*grid), grid
