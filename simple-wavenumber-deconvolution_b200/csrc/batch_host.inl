@@ -173,7 +173,8 @@ static int rtm_batch_once(swd_ctx *ctx, const swd_shot *shots, const float *cons
     // per step of four shots without / with: 2251 x 1101 313.6 / 276.1, 2001 x 1001 256.5 / 229.0, 1901
     // x 951 217.9 / 223.0; of eight 1201 x 601 200.7 / 210.7)
     const double work = 12.0 * sizeof(float) * (double)ctx->ntx * ctx->ldz;   // of a shot's backward step
-    const int ahead = work > 0.75 * (double)ctx->l2_bytes && nb * work > 3.0 * (double)ctx->l2_bytes ? 1 : 0;
+    const int ahead = work > 0.75 * (double)ctx->l2_bytes && nb * work > 3.0 * (double)ctx->l2_bytes &&
+                      ahead_fits(ctx->ldz, 12, ctx->l2_bytes) ? 1 : 0;
     a.ahead = ahead;
     a.g = make_geo(ctx);
     a.c = make_cpml(ctx);

@@ -15,6 +15,7 @@
 #include <cuda_fp16.h>
 #include <cuda_bf16.h>
 #include <stdint.h>
+#include "rules.h"
 
 namespace swd {
 
@@ -655,9 +656,8 @@ __device__ __forceinline__ void cell4(int &x, int &z0)
 // 131.8 / 116.4, 2501 x 1203 66.8 / 63.7, 2001 x 1001 44.8 / 44.4, 1601 x 801 26.3 / 27.7; scattered
 // field 4001 x 1601 150.8 / 130.1, 1601 x 801 31.6 / 32.5; field and twin 4001 x 1601 127.7 / 106.4.
 // 24 to 64 columns ahead give the same, 1 column ahead half of it, from 320 on lines are evicted
-// again before they are read.  Its own instantiations (stencil order 4): as a branch it cost the grids
+// again before they are read (ahead_fits bounds that by cells).  Its own instantiations (stencil order 4): as a branch it cost the grids
 // that stay in L2 3% in registers.
-constexpr int AHEAD_COLS = 40;
 __device__ __forceinline__ size_t ahead_cell(const Geo &g, int x, int z0)
 {
     return (size_t)min(x + AHEAD_COLS, g.ntx - 1) * g.ldz + z0;

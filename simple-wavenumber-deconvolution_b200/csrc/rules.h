@@ -24,6 +24,14 @@ inline bool march_index_fits(int ntx, int ldz) { return (long long)ntx * ldz <= 
 // 16000 x 400 1.17 92.1 / 81.4, 20000 x 300 1.48 106.2 / 84.1, 40000 x 160 2.38 184.7 / 125.1.
 inline bool march_pays(size_t frame_tasks, long long cells) { return (long long)frame_tasks * (17 + 7) * 128 <= cells; }
 
+// Whether operands prefetched into L2 AHEAD_COLS columns ahead are still there when they are read: what a
+// pass of so many arrays touches in those columns is at most a quarter of the L2.  RTM backward step,
+// us, without / with: 20000 rows 128.8 / 137.0, 15000 rows 126.0 / 127.5, 9000 rows 126.3 / 120.6; forward
+// step (6 arrays) 60000 rows 100.4 / 112.5, 30000 rows 78.4 / 73.8; scattered field (10 arrays a launch)
+// 30000 rows 152.0 / 175.2, 20000 rows and 3000 columns 1016 / 976, 10000 rows 125.2 / 115.0.
+constexpr int AHEAD_COLS = 40;
+inline bool ahead_fits(int ldz, int arrays, size_t l2_bytes) { return (size_t)AHEAD_COLS * ldz * sizeof(float) * arrays <= l2_bytes / 4; }
+
 // Whether a smoothing window of this half width works on a tile of doubles in shared memory, on a grid
 // of so many blocks (32 x 8 cells).  Wider windows leave an SM fewer blocks and so too few warps for the
 // additions' latency, first where the grid is one wave or little more.  Call with the tile / taps from

@@ -1619,7 +1619,7 @@ static int run_forward(swd_ctx *ctx, FwdJob &J, ShotPlan &P)
     const int nw = J.twin ? 2 : 1;
     // (the marches and the on-chip loops take none of these; one field's step kernels gain from
     // 5.5 M cells on, 4001 x 1601 69.0 -> 62.1 us, two fields' from 2.8 M)
-    a.ahead = streams_hbm(ctx, nw == 2 ? 12 : 6) ? 1 : 0;
+    a.ahead = streams_hbm(ctx, nw == 2 ? 12 : 6) && ahead_fits(ctx->ldz, nw == 2 ? 10 : 6, ctx->l2_bytes) ? 1 : 0;
     ResPlan rp;
     // Born modelling on the chip, in pieces of the checkpoint interval (RES_PIECE)
     if (a.dkappa && nw == 2 && !a.s0_out && !a.ds.buf && !a.strips.buf && (!a.ck.every || a.ck.every >= RES_PIECE) &&
@@ -2564,7 +2564,7 @@ static int rtm_backward_part(swd_ctx *ctx, const swd_shot *shot, const float *da
     }
     BwdArgs b;
     memset(&b, 0, sizeof b);
-    b.ahead = streams_hbm(ctx, 12) ? 1 : 0;
+    b.ahead = streams_hbm(ctx, 12) && ahead_fits(ctx->ldz, 12, ctx->l2_bytes) ? 1 : 0;
     b.g = make_geo(ctx);
     b.c = make_cpml(ctx);
     b.vp = F(ctx->vp);

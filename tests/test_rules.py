@@ -10,6 +10,7 @@ WRAP = """
 #include "rules.h"
 extern "C" {
 int bands_apart(int ntz, int pmlc, int Lc) { return swd::strip_bands_apart(ntz, pmlc, Lc); }
+int ahead_fits(int ldz, int arrays, size_t l2) { return swd::ahead_fits(ldz, arrays, l2); }
 int march_pays(size_t frame_tasks, long long cells) { return swd::march_pays(frame_tasks, cells); }
 int smooth_tile(int window, long long blocks) { return swd::smooth_tile(window, blocks); }
 long long smooth_smem(int window) { return swd::smooth_smem(window); }
@@ -94,3 +95,12 @@ def test_march_wants_little_frame(rules):
         assert pays(*grid), grid
     for grid in ((16000, 400, 30, 33), (30000, 200, 10, 33), (60000, 100, 10, 33), (60, 90000, 10, 33)):
         assert not pays(*grid), grid
+
+
+def test_reads_ahead_stay_in_l2(rules):
+    """126 MB of L2: grids of the usual depth read ahead in every pass, tall ones only with few arrays."""
+    rules.ahead_fits.argtypes = [C.c_int, C.c_int, C.c_size_t]
+    fits = lambda ldz, arrays: bool(rules.ahead_fits(ldz, arrays, 132644864))
+    assert fits(1696, 12) and fits(4096, 12) and fits(30080, 6)
+    assert not fits(20096, 12) and fits(20096, 10) and not fits(30080, 10) and not fits(60096, 6)
+    assert not rules.ahead_fits(64, 6, 0)   # an L2 of unknown size
