@@ -217,6 +217,8 @@ def algorithmic_bytes(kernel, w, cp, strip_len, r_n, strip_esz=4):
         return 48 * N + 16 * x_v
     if kernel == "fwd_p2":     # pressures of both (shared ck); both fields' traces; the well columns of both
         return 36 * N + 16 * x_p + 8 * r_n + 8 * w.extra.get("well_columns", 1) * w.ntz
+    if kernel == "fwd_march":  # one launch per forward step of large grids: p, vx, vz r/w, cbx, cbz, ck, CPML, strips
+        return 36 * N + 8 * (x_v + x_p) + strip_esz * strip_len + 4 * r_n
     if kernel == "fwd_step":   # one fused launch per forward step: p, vx, vz r/w, vp, rho, CPML, strips
         return 32 * N + 8 * (x_v + x_p) + strip_esz * strip_len + 4 * r_n
     if kernel == "bwd_step":   # one fused launch per backward step: receiver 24N, material 8N, source 24Ni, FP64 image 32Ni
@@ -384,6 +386,8 @@ def run_ours(args, rank, world, dist):
     per_launch = {k: ms / n for k, (ms, n) in prof.items() if n}
     if E.get_option(swd.OPT_BWD_BY_KIND):   # profile slots 2, 3 hold k_bwd_v, k_bwd_p
         per_launch = {{"bwd_1": "bwd_v", "bwd_2": "bwd_p"}.get(k, k): v for k, v in per_launch.items()}
+    if "fwd_step" in per_launch and args.path != 1:   # the plain path's forward steps of large grids
+        per_launch["fwd_march"] = per_launch.pop("fwd_step")
     # Kernel durations: the whole-pass events (around the graph replays, nothing inside the
     # captured steps) give the time of one forward / backward time step; a probe copy of one
     # chunk brackets the kernels of its middle step, which inflates each by the event-node
@@ -395,12 +399,12 @@ def run_ours(args, rank, world, dist):
         if ps in per_launch and k1 in per_launch and k2 in per_launch:
             t, a1, a2 = per_launch[ps], per_launch[k1], per_launch[k2]
             live[k1], live[k2] = t * a1 / (a1 + a2), t * a2 / (a1 + a2)
-    for k in ("fwd_step", "bwd_step"):   # fused path: one launch per step
-        ps = k.replace("_step", "_pass_step")
+    for k in ("fwd_step", "bwd_step", "fwd_march"):   # one launch per step
+        ps = k[:3] + "_pass_step"
         if ps in per_launch and k in per_launch:
             live[k] = per_launch[ps]
     launches_per_shot = {"fwd_v": nt, "fwd_p": nt, "bwd_1": nt - 1, "bwd_2": nt - 1, "bwd_v": nt - 1, "bwd_p": nt - 1,
-                         "fwd_step": nt, "bwd_step": nt - 1}
+                         "fwd_step": nt, "bwd_step": nt - 1, "fwd_march": nt}
     dom = max(live, key=lambda k: live[k] * launches_per_shot[k])
     peak, src = peaks()
     ab = algorithmic_bytes(dom, w, cp, slen, r_n, 4 if strips == "f32" else 2)

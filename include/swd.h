@@ -254,12 +254,12 @@ int swd_rtm_batch(swd_ctx *ctx, int nshots, const swd_shot *shots, const float *
  *                 its adjoint from 8 steps per checkpoint on) on grids whose wavefields fit in the
  *                 SMs' shared memory and registers run as one cooperative launch that keeps the
  *                 fields on the chip between steps (stencil order 4, the other options at their
- *                 defaults, no profiling).  The same results bit for bit.  0: the step kernels. */
+ *                 defaults).  The same results bit for bit.  0: the step kernels. */
 #define SWD_OPT_RESIDENT 13
 /* SWD_OPT_MARCH 1 (default): on grids whose fields fill the device's L2, the forward passes of one
  *                 wavefield (RTM, modelling without a twin) run each time step as one sweep along x
  *                 that makes both half steps (stencil order 4, the other options at their defaults,
- *                 no profiling, an absorbing frame that is not most of the grid).  The same results bit for bit.  0: the step kernels. */
+ *                 an absorbing frame that is not most of the grid).  The same results bit for bit.  0: the step kernels. */
 #define SWD_OPT_MARCH 14
 /* SWD_OPT_RESIDENT_STOP n (default 0: off), for tests of the recovery from an on-chip pass in which a
  *                 wait for a neighbouring tile gave up (after a second or two): n > 0 ends the passes
@@ -346,7 +346,8 @@ int swd_decon(swd_ctx *ctx, const swd_decon_params *p, const float *migreal,
  * swd_profile(ctx, every): bracket each kernel launch of every `every`-th time step with
  * CUDA events on the context stream (0 disables).  swd_profile_read fills, per kernel id
  * (0 forward-v, 1 forward-p, 2 backward-1, 3 backward-2 of the plain path; 4 forward step,
- * 5 backward step of the fused path; 6 / 7 whole forward / backward time steps, i.e. a pass
+ * 5 backward step made by one launch (the fused path, marching forward steps) or inside one (on-chip
+ * passes, divided by their steps); 6 / 7 whole forward / backward time steps, i.e. a pass
  * divided by its steps; 8 / 9 the two adjoint kernels of swd_born_adjoint and 10 its whole
  * adjoint time step), the summed milliseconds and the
  * number of timed launches, and clears them.  swd_launch_count is the number of kernels the

@@ -1283,7 +1283,7 @@ static int run_steps(swd_ctx *ctx, swd_ctx::StepGraph &G, const void *key, size_
 // Whether the context's options ask for nothing but the default step kernels (with graphs or not).
 static bool default_steps(const swd_ctx *c)
 {
-    return c->path == SWD_PATH_PLAIN && !c->autotune && !c->use_tma && !c->use_staged && !c->use_pdl && c->use_lean && c->prof_every == 0;
+    return c->path == SWD_PATH_PLAIN && !c->autotune && !c->use_tma && !c->use_staged && !c->use_pdl && c->use_lean;
 }
 
 // ---- on-chip time loops (resident.cuh) ---------------------------------------------------
@@ -1372,7 +1372,14 @@ static int run_resident(swd_ctx *ctx, ResArgs &a, const ResPlan &p, int mode, bo
     a.stop = ctx->res_stop > 0 ? 1 : ctx->res_stop;
     if (ctx->res_stop > 0) a.nsteps = std::min(a.nsteps, ctx->res_stop);
     ctx->res_epoch += (unsigned)a.nsteps + 1u;
-    if (res_launch(a, p, mode, ctx->stream) != cudaSuccess) {
+    cudaError_t e;
+    {
+        // the launch is all of its steps (profiling ids 4 and 6, backward 5 and 7)
+        const bool prof = ctx->prof_every > 0;
+        ProfScope pass(ctx, mode == 1 ? 7 : 6, prof, a.nsteps), step(ctx, mode == 1 ? 5 : 4, prof, a.nsteps);
+        e = res_launch(a, p, mode, ctx->stream);
+    }
+    if (e != cudaSuccess) {
         cudaGetLastError();
         ctx->use_resident = 0;
         return SWD_OK;
@@ -1532,17 +1539,19 @@ static int run_forward_march(swd_ctx *ctx, const FwdArgs &a, ShotPlan &P, bool *
     m.w = march_wave(ctx, 0, 0);
     const int nwarp = (int)tasks.size();
     CK(cudaFuncSetAttribute(k_march_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, MARCH_FWD_SMEM));
-    auto launch = [&](int k, cudaEvent_t *) {
+    auto launch = [&](int k, cudaEvent_t *ev) {
         MFwdArgs b = m;
         b.itoff = k;
         b.w = march_wave(ctx, 0, k & 1);   // chunks start at even steps
+        if (ev) cudaEventRecordWithFlags(ev[0], ctx->stream, cudaEventRecordExternal);
         k_march_fwd<<<nwarp, 32, MARCH_FWD_SMEM, ctx->stream>>>(b);
+        if (ev) cudaEventRecordWithFlags(ev[1], ctx->stream, cudaEventRecordExternal);
         if (nlist && k == GRAPH_K - 1) k_march_encode<<<dim3(nlist, GRAPH_K), 128, 0, ctx->stream>>>(en);
     };
     struct { MFwdArgs m; MEncodeArgs e; int nlist, nwarp; } key;
     memset(&key, 0, sizeof key);
     key.m = m; key.e = en; key.nlist = nlist; key.nwarp = nwarp;
-    const int kid[1] = {0};
+    const int kid[1] = {4};
     CKR(run_steps(ctx, ctx->gfwd, &key, sizeof key, 0, +1, a.nt, 1, kid, launch));
     if (nlist && a.nt % GRAPH_K) {   // the steps after the last chunk
         k_march_encode<<<dim3(nlist, a.nt % GRAPH_K), 128, 0, ctx->stream>>>(en);
