@@ -427,29 +427,31 @@ constexpr int GATHER_NTHR = 256;
 __global__ void __launch_bounds__(GATHER_NTHR) k_decon_gather(DeconGeo g, const float *__restrict__ winout, const float *__restrict__ coefr,
                                                               float *__restrict__ dec, float *__restrict__ coef)
 {
-    const int px = blockIdx.x, pz = blockIdx.y * GATHER_NTHR + threadIdx.x;
-    if (pz >= g.nz) return;
+    const int px = blockIdx.x;
     const int nout = g.outwinx * g.outwinz;
     // windows a (x) with a*stepwinx - halfoutwx <= px <= a*stepwinx - halfoutwx + outwinx - 1
     int alo = px + g.halfoutwx - g.outwinx + 1;
     alo = alo <= 0 ? 0 : (alo + g.stepwinx - 1) / g.stepwinx;
     const int ahi = min((px + g.halfoutwx) / g.stepwinx, g.stepnumx - 1);
-    int blo = pz + g.halfoutwz - g.outwinz + 1;
-    blo = blo <= 0 ? 0 : (blo + g.stepwinz - 1) / g.stepwinz;
-    const int bhi = min((pz + g.halfoutwz) / g.stepwinz, g.stepnumz - 1);
-    float acc = 0.f, cacc = 0.f;
-    for (int a = alo; a <= ahi; a++)
-        for (int b = blo; b <= bhi; b++) {
-            const int ixx = px - (a * g.stepwinx - g.halfoutwx), izz = pz - (b * g.stepwinz - g.halfoutwz);
-            const int ipc = ixx * g.outwinz + izz;
-            const float cr = __ldg(coefr + ipc);
-            const float v = __ldg(winout + (size_t)(a * g.stepnumz + b) * nout + ipc);
-            acc = (float)((double)acc + (double)v * (double)cr);
-            cacc = cacc + cr;
-        }
-    const size_t i = (size_t)px * g.nz + pz;
-    dec[i] = acc;
-    coef[i] = cacc;
+    // (a grid has at most 65,535 block rows)
+    for (int pz = blockIdx.y * GATHER_NTHR + threadIdx.x; pz < g.nz; pz += gridDim.y * GATHER_NTHR) {
+        int blo = pz + g.halfoutwz - g.outwinz + 1;
+        blo = blo <= 0 ? 0 : (blo + g.stepwinz - 1) / g.stepwinz;
+        const int bhi = min((pz + g.halfoutwz) / g.stepwinz, g.stepnumz - 1);
+        float acc = 0.f, cacc = 0.f;
+        for (int a = alo; a <= ahi; a++)
+            for (int b = blo; b <= bhi; b++) {
+                const int ixx = px - (a * g.stepwinx - g.halfoutwx), izz = pz - (b * g.stepwinz - g.halfoutwz);
+                const int ipc = ixx * g.outwinz + izz;
+                const float cr = __ldg(coefr + ipc);
+                const float v = __ldg(winout + (size_t)(a * g.stepnumz + b) * nout + ipc);
+                acc = (float)((double)acc + (double)v * (double)cr);
+                cacc = cacc + cr;
+            }
+        const size_t i = (size_t)px * g.nz + pz;
+        dec[i] = acc;
+        coef[i] = cacc;
+    }
 }
 
 }  // namespace swd

@@ -788,10 +788,12 @@ __global__ void __launch_bounds__(256) k_material_segs(Mat m, Mat m1, const floa
 // thread per frame cell
 __global__ void k_pml_x(float *v, int ntx, int ntz, int pml)
 {
-    const int iz = blockIdx.x * blockDim.x + threadIdx.x + pml, k = blockIdx.y;
+    const int iz = blockIdx.x * blockDim.x + threadIdx.x + pml;
     if (iz > ntz - pml - 1) return;
-    if (k < pml) v[(size_t)k * ntz + iz] = v[(size_t)pml * ntz + iz];
-    else v[(size_t)(ntx - 2 * pml + k) * ntz + iz] = v[(size_t)(ntx - pml - 1) * ntz + iz];
+    for (int k = blockIdx.y; k < 2 * pml; k += gridDim.y) {   // (at most 65,535 block rows)
+        if (k < pml) v[(size_t)k * ntz + iz] = v[(size_t)pml * ntz + iz];
+        else v[(size_t)(ntx - 2 * pml + k) * ntz + iz] = v[(size_t)(ntx - pml - 1) * ntz + iz];
+    }
 }
 __global__ void k_pml_z(float *v, int ntx, int ntz, int pml)
 {
@@ -1874,7 +1876,7 @@ static int decon_geo(const swd_decon_params *p, DeconGeo &g)
     return SWD_OK;
 }
 
-static dim3 gather_grid(const DeconGeo &g) { return dim3(g.nx, (g.nz + GATHER_NTHR - 1) / GATHER_NTHR); }
+static dim3 gather_grid(const DeconGeo &g) { return dim3(g.nx, std::min((g.nz + GATHER_NTHR - 1) / GATHER_NTHR, 65535)); }
 
 // Launch shape of the persistent window kernel (staged transforms or the iterative option): a
 // 96 KB shared chunk when staged, else the buffer in shared memory; as many CTAs as are
@@ -2906,7 +2908,7 @@ int swd_smooth(swd_ctx *ctx, int ntx, int ntz, int pml, int window, float *vp)
         k_smooth<false><<<grid, block, 0, ctx->stream>>>(F(a), F(b), D(cf), ntx, ntz, pml, window);
     }
     if (pml > 0) {
-        k_pml_x<<<dim3((ntz - 2 * pml + 127) / 128, 2 * pml), 128, 0, ctx->stream>>>(F(b), ntx, ntz, pml);
+        k_pml_x<<<dim3((ntz - 2 * pml + 127) / 128, std::min(2 * pml, 65535)), 128, 0, ctx->stream>>>(F(b), ntx, ntz, pml);
         k_pml_z<<<(unsigned)(((size_t)ntx * 2 * pml + 127) / 128), 128, 0, ctx->stream>>>(F(b), ntx, ntz, pml);
     }
     CK(cudaGetLastError());
