@@ -174,3 +174,23 @@ def test_on_chip_pass_without_room_for_its_exchange_words(swd):
     n0 = E.launch_count()
     assert np.array_equal(E.forward(s, rick), ref)
     assert E.launch_count() - n0 < nt                   # on the chip again
+
+
+def test_decon_without_a_context_frees_what_it_took(swd):
+    """The same result as with a context, arrays on the device and on the host, and no memory kept; on a
+    nearly full device by the FFT windows."""
+    job = Decon(swd)
+    none = type("NoContext", (), {"_h": None, "_ck": staticmethod(lambda rc: rc == 0 or pytest.fail(f"error {rc}"))})
+    E = swd.Engine(64, 64, 8, 4, 5.0, 5.0, 5e-4, 64)
+    ref = job(E)
+    E.close()
+    job(none)
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    assert np.array_equal(job(none), ref)
+    with Filled(152 * MB):
+        assert rel_l2(job(none), ref) < 2e-5
+    host = swd.decon(*[t.cpu().numpy() for t in job.ins], (79, 79), (79, 79), (24, 24), 1e-3, psf_interp=1)[0]
+    assert np.array_equal(host, ref)
+    torch.cuda.synchronize()
+    assert torch.cuda.mem_get_info()[0] == free
