@@ -326,7 +326,9 @@ typedef struct {
     int psf_interp;
     /* 0: the window's transform buffer in shared memory when it fits (FX*FZ*8 bytes up to about
      * 200 KB, e.g. 158 x 158), otherwise in a global-memory workspace with each transform pass
-     * staged through shared memory (same arithmetic, same bits); 1: always the workspace */
+     * staged through shared memory (same arithmetic, same bits); 1: always the workspace.  Of the
+     * FFT windows only: windows that run as matrix products (the direct division wherever their
+     * tables fit in shared memory) use neither, and give the same bits either way. */
     int workspace;
     /* Iterative regularised deconvolution (project option: the reference parses reg_eps and its
      * parameter file lists an L2 coefficient and an iteration count, kkdecon_acoustic/
