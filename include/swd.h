@@ -235,7 +235,8 @@ int swd_rtm_batch(swd_ctx *ctx, int nshots, const swd_shot *shots, const float *
  *                 context.  Every variant gives the same images bit for bit, so only the speed of
  *                 the first few shots depends on the order.  Setting the option restarts the tuning;
  *                 while it is on it overrides SWD_OPT_TMA, SWD_OPT_STAGED and SWD_OPT_BWD_BY_KIND
- *                 for those passes.  0 (default): the options as set.
+ *                 for those passes, and SWD_OPT_RESIDENT and SWD_OPT_MARCH are off: it tunes the step
+ *                 kernels, which are the slower way where those two apply.  0 (default): the options as set.
  * SWD_OPT_TUNED_FWD / SWD_OPT_TUNED_BWD (read only): the chosen variant (forward: 1 TMA velocity
  *                 + 2 staged pressure, 8 / 16 pressure kernel at 4 / 6 blocks per SM, 32 velocity
  *                 kernel at 6; backward: 1 TMA velocity, 4 reference pairing, 8 / 16 at 4 / 6
