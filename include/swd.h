@@ -265,8 +265,9 @@ int swd_rtm_batch(swd_ctx *ctx, int nshots, const swd_shot *shots, const float *
 /* SWD_OPT_RESIDENT_STOP n (default 0: off), for tests of the recovery from an on-chip pass in which a
  *                 wait for a neighbouring tile gave up (after a second or two): n > 0 ends the passes
  *                 after n steps with the first tile reporting that it gave up, -1 keeps the first
- *                 tile from starting, so that the others' waits run out.  The call then runs
- *                 again with the step kernels (same results) and SWD_OPT_RESIDENT reads 0. */
+ *                 tile from starting, so that the others' waits run out, -2 makes the runtime
+ *                 refuse the launch.  The call then runs (again) with the step kernels (same
+ *                 results) and SWD_OPT_RESIDENT reads 0. */
 #define SWD_OPT_RESIDENT_STOP 15
 int swd_set_option(swd_ctx *ctx, int option, int value);
 int swd_get_option(swd_ctx *ctx, int option, int *value);

@@ -421,7 +421,7 @@ int swd_set_option(swd_ctx *ctx, int option, int value)
             ctx->use_resident = value;
             return SWD_OK;
         case SWD_OPT_RESIDENT_STOP:
-            if (value < -1) return fail(ctx, SWD_ERR_ARG, "SWD_OPT_RESIDENT_STOP takes -1, 0 or a number of steps");
+            if (value < -2) return fail(ctx, SWD_ERR_ARG, "SWD_OPT_RESIDENT_STOP takes -2, -1, 0 or a number of steps");
             ctx->res_stop = value;
             return SWD_OK;
         case SWD_OPT_LEAN:

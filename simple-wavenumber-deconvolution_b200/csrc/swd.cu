@@ -1371,7 +1371,9 @@ static int run_resident(swd_ctx *ctx, ResArgs &a, const ResPlan &p, int mode, bo
     a.GX = p.GX;
     a.GZ = p.GZ;
     a.epoch = ctx->res_epoch;
-    a.stop = ctx->res_stop > 0 ? 1 : ctx->res_stop;
+    a.stop = ctx->res_stop > 0 ? 1 : ctx->res_stop == -1 ? -1 : 0;
+    ResPlan q = p;
+    if (ctx->res_stop == -2) q.GX = 1 << 20;   // more blocks than fit at once: the runtime refuses the launch
     if (ctx->res_stop > 0) a.nsteps = std::min(a.nsteps, ctx->res_stop);
     ctx->res_epoch += (unsigned)a.nsteps + 1u;
     cudaError_t e;
@@ -1379,7 +1381,7 @@ static int run_resident(swd_ctx *ctx, ResArgs &a, const ResPlan &p, int mode, bo
         // the launch is all of its steps (profiling ids 4 and 6, backward 5 and 7)
         const bool prof = ctx->prof_every > 0;
         ProfScope pass(ctx, mode == 1 ? 7 : 6, prof, a.nsteps), step(ctx, mode == 1 ? 5 : 4, prof, a.nsteps);
-        e = res_launch(a, p, mode, ctx->stream);
+        e = res_launch(a, q, mode, ctx->stream);
     }
     if (e != cudaSuccess) {
         cudaGetLastError();

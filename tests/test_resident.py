@@ -246,11 +246,16 @@ def test_waits_that_run_out(swd, name):
     _gives_up(swd, "smallest", name, (-1,))
 
 
+@pytest.mark.parametrize("name", GIVE_UP)
+def test_refused_launch_runs_the_step_kernels(swd, name):
+    _gives_up(swd, "z_one_row_left", name, (-2,))
+
+
 def test_stop_option(swd):
     E = _engine(swd, 20, 20, 10, 16, 1)[0]
     assert E.get_option(swd.OPT_RESIDENT_STOP) == 0
     with pytest.raises(swd.SwdError):
-        E.set_option(swd.OPT_RESIDENT_STOP, -2)
+        E.set_option(swd.OPT_RESIDENT_STOP, -3)
 
 
 def test_error_after_a_pass_that_gave_up(swd):
