@@ -1322,11 +1322,11 @@ struct InCall {
 
 // Whether the context's options ask for nothing but the default step kernels and the grid's
 // wavefields fit on the chip; plan receives the tiling for nw wavefields.  The plain kernels keep
-// every other case: larger grids, other stencil lengths, 16-bit strips, the kernel variants
-// the options select, and calls beside another one on the device: engines of a pool overlap
-// their step kernels, but these launches would have to take turns (us per step and shot, on the chip / step kernels:
-// RTM 401 x 201 one engine 9.4 / 17.0, two 9.3 / 9.8, three 9.3 / 7.2; 801 x 401 13.7 / 19.4, 13.6 /
-// 12.6, 13.5 / 9.9; Born and adjoint 801 x 401 23.9 / 29.1, 23.0 / 20.1, 22.7 / 15.9).  Same bits.
+// every other case: larger grids, other stencil lengths, 16-bit strips, the kernel variants the options
+// select, and calls beside another one on the device: engines of a pool overlap their step kernels,
+// but these launches would have to take turns (us per step and shot, on the chip in turns / step
+// kernels: RTM 401 x 201 one engine 9.4 / 17.0, two 9.3 / 9.8, three 9.3 / 7.2; 801 x 401 13.7 / 19.4,
+// 13.6 / 12.6, 13.5 / 9.9; Born and adjoint 801 x 401 23.9 / 29.1, 23.0 / 20.1, 22.7 / 15.9).  Same bits.
 static bool resident_plan(const swd_ctx *c, int nw, ResPlan *plan, bool born = false)
 {
     if (calls_on(c->dev) > 1) return false;
